@@ -113,8 +113,9 @@ typedef struct {
     double  inner_tol;        /* mixed form: relative tolerance of each FP32 sweep */
     int32_t max_sweeps;       /* mixed form: cap on refinement sweeps */
     int32_t check_every;      /* Krylov iterations between host convergence checks (systems
-                                 above 2^18 rows; smaller FP64 BiCGStab solves run in one
-                                 persistent launch and test every iteration) */
+                                 too large for the SMs; an FP64 BiCGStab solve of up to
+                                 about 800,000 rows runs resident on them and tests every
+                                 iteration) */
     double  timeout_s;        /* host wall-clock limit of one solve (<= 0: none) */
     int32_t inner_adaptive;   /* mixed form: relax the last sweeps' inner tolerance to what the outer
                                  tolerance still needs (never tighter than inner_tol) */
@@ -346,9 +347,8 @@ mhfem_status mhfem_get_stream(mhfem_t h, void** stream);
 mhfem_status mhfem_time_kernel(mhfem_t h, int32_t kernel, int32_t reps, double* ms_per_launch,
                                double* bytes_per_launch, double* flops_per_launch);
 
-/* Check of the bounded grid barrier that the small-system FP64 BiCGStab
- * (systems of at most 2^18 rows, one cooperative launch per solve) places
- * between its phases.  One cooperative launch of `ctas` CTAs on `device`
+/* Check of the bounded grid barrier that the persistent solves (the resident
+ * FP64 BiCGStab, the GMRES of at most 2^18 rows) place between their phases.  One cooperative launch of `ctas` CTAs on `device`
  * passes through the barrier once, every wait polling at most `max_polls`
  * times; CTA `skip_cta` (none if negative) never arrives, so the others'
  * waits run out, set the failure flag and return -- the kernel ends without
@@ -418,7 +418,7 @@ mhfem_status mhfem_learned_status(mhfem_t h, int32_t* trained_steps, double* las
  * solve and a system with any other index is refused with
  * MHFEM_ERR_INVALID_ARGUMENT (nothing else runs).
  * All work vectors live in one static device array of fixed size (about
- * 17 MB), so systems with more than MHFEM_NOALLOC_MAX_ROWS rows are
+ * 13 MB), so systems with more than MHFEM_NOALLOC_MAX_ROWS rows are
  * rejected with MHFEM_ERR_INVALID_ARGUMENT.  Under CUDA's default lazy module
  * loading that array is committed on a device at the FIRST call there (which
  * looks its address up with cudaGetSymbolAddress and may synchronize the
@@ -427,10 +427,9 @@ mhfem_status mhfem_learned_status(mhfem_t h, int32_t* trained_steps, double* las
  * initialization, before any stream capture.  Every call shares the array:
  * calls that overlap on the GPU (other streams, other threads) race and must
  * be serialized by the caller.
- * The solve is the persistent small-system BiCGStab that mhfem_solve runs
- * for systems of this size (one cooperative launch per chunk of up to 256
- * iterations, the convergence test in every iteration), so the two entry
- * points return the same iterates.
+ * The solve is the resident BiCGStab that mhfem_solve runs for systems of
+ * this size (one launch per chunk of up to 256 iterations, the convergence
+ * test in every iteration), so the two entry points return the same iterates.
  * The call blocks until the solve ends: at most max_iter iterations, and at
  * most timeout_s seconds of wall-clock time when timeout_s > 0 (checked
  * between chunks, after the queued work has drained; then

@@ -1,0 +1,104 @@
+"""The FP64 BiCGStab resident on the SMs (csrc/k_resident.cu) at the edges of
+its forms, against the oracle: one CTA, clusters of 2 to 16 with a partial
+last block of rows, the largest cluster and the first grid, both sides of the
+size where phase B stops forming the neighbours' s, the sizes where the ELL
+words and then x leave shared memory, and the last resident system and the
+first one above it; run-time and compile-time widths.
+
+The bar is the parity tests': both sides solve to 1e-13, the states agree
+within 1e-10.
+"""
+import numpy as np
+import pytest
+
+from helpers import diffusion3d_n2, rel_err
+from mhfem import problems
+from oracle.oracle import OracleModel
+
+pytestmark = pytest.mark.gpu
+
+TOL_STATE = 1e-10
+
+# (model, N): the row count in the comment
+SIZES = [
+    ("heat2d", 2),           # 16: one CTA
+    ("heat2d", 6),           # 120
+    ("heat2d", 7),           # 161: a cluster of 2
+    ("heat2d", 17),          # 901: 8, the last block partial
+    ("heat2d", 51),          # 7,905: the largest cluster
+    ("heat2d", 53),          # 8,533: the smallest grid
+    ("heat2d", 162),         # 79,056: neighbours' s recomputed
+    ("heat2d", 164),         # 81,016: s published
+    ("heat2d", 345),         # 357,765: ELL words streamed
+    ("heat2d", 520),         # 812,240: x in memory, the largest resident system
+    ("heat2d", 523),         # 821,633: five kernels
+    ("diffusion3d", 3),      # width 6: 378
+    ("diffusion3d", 13),     # 27,378
+    ("diffusion3d", 29),     # 297,714: streamed
+    ("diffusion3d_box", 9),  # width 10: 2,430
+    ("diffusion3d_box", 36),  # 143,856
+    ("diffusion3d_box", 50),  # 382,500: streamed
+    ("adr2d", 15),           # width 9: 1,410
+    ("adr2d", 120),          # 86,880
+    ("adr2d", 240),          # 346,560: streamed
+    ("diffusion3d_n2", 6),   # width 13: 5,616
+    ("diffusion3d_n2", 20),  # 196,800
+    ("box3d_lumped", 10),    # a lumped cuboid system
+]
+
+
+def _problem(name, N):
+    if name == "diffusion3d_n2":
+        p = diffusion3d_n2(N)
+    elif name == "box3d_lumped":
+        p = problems.diffusion3d_box(N=N, steps=2, lumping=True)
+    else:
+        p = problems.WORKLOADS[name](N=N, steps=2)
+    p.tol = 1e-13
+    return p
+
+
+@pytest.mark.parametrize("name,N", SIZES)
+def test_resident_solve_against_oracle(name, N):
+    p = _problem(name, N)
+    s = problems.make_solver(p)
+    m = OracleModel.from_problem(p)
+    t = 0.0
+    for _ in range(1 if s.F * p.n > 100000 else 2):
+        st = s.step(t, p.dt)
+        m.step(t, p.dt, 1e-13)
+        assert st["residual"] < 1e-13
+        t += p.dt
+    zf, zk = s.state()
+    assert rel_err(zf, m.Z_iF) < TOL_STATE
+    assert rel_err(zk, m.Z_iK) < TOL_STATE
+    s.close()
+
+
+@pytest.mark.parametrize("name,N", [("heat2d", 40), ("heat2d", 100), ("diffusion3d", 29)])
+def test_resident_solve_continues_after_a_chunk(name, N):
+    """A time step 400 times as long takes more iterations than one launch
+    runs (256): the solve goes on from the state the launch left, in the
+    cluster, the grid and the streamed form."""
+    p = _problem(name, N)
+    p.dt *= 400.0
+    s = problems.make_solver(p)
+    m = OracleModel.from_problem(p)
+    s.step(0.0, p.dt)
+    m.step(0.0, p.dt, 1e-13)
+    # two solutions with residuals of 1e-13 differ by at most 2e-13 times the
+    # condition number, which is below 24 N^2 dt (heat) and 5e4 here
+    assert rel_err(s.state()[0], m.Z_iF) < 1e-8
+    s.close()
+
+
+def test_resident_solve_iteration_cap():
+    p = _problem("heat2d", 64)
+    s = problems.make_solver(p, max_iter=7)
+    with pytest.raises(Exception, match="7 iterations"):
+        s.step(0.0, p.dt)
+    s.setup(tol=1e-12, max_iter=1000)
+    s.setInitialCondition(p.Z0)
+    assert s.step(0.0, p.dt)["residual"] < 1e-12
+    assert np.isfinite(s.state()[0]).all()
+    s.close()

@@ -785,29 +785,7 @@ __global__ void __launch_bounds__(KB) k_update_p(int64_t rows, T* p, const T* r,
     }
 }
 
-// ---- small systems: one persistent launch per chunk of iterations ----------------
-//
-// A system of a few ten thousand rows (the 128^2 heat-equation workload:
-// 49,408 rows, about 2 MB of matrix and vectors, all L2-resident) leaves the
-// five-kernel iteration bound by launch and drain latency: about 30 us per
-// iteration for a few microseconds of memory traffic.  Here one cooperative
-// launch (every CTA resident) runs a chunk of iterations:
-//  - an iteration is three phases separated by grid barriers (below:
-//    k_bicgstab_small), the p and s updates being formed where they are
-//    gathered; measured on the 128^2 system: 24.7 us per iteration against
-//    26.8 us with five phases and 30.6 us for the five-kernel iteration;
-//  - each reduction's per-CTA partials are summed by every CTA itself, in
-//    the same fixed order, so every CTA holds the same scalars (in shared
-//    memory) with no last-block step, and the result is deterministic;
-//  - the convergence test runs every iteration, as in the reference's loop
-//    (the five-kernel path tests every check_every iterations);
-//  - a thread owns the same rows in every phase, so its own rows need no
-//    synchronization; values of other CTAs' rows (the SpMV gathers, the
-//    partials) are loaded past L1 (ld.global.cg), which is not coherent
-//    between SMs; the matrix, constant during the solve, stays in L1.
-// Every barrier wait is bounded: a CTA that polls kBarrierPolls times
-// records the failure in *bar_err and returns, and the others then fail
-// their next wait at once.
+// ---- check of the bounded grid wait ------------------------------------------------
 
 // Check of the bounded barrier: every CTA but `skip` (none if negative)
 // arrives once and reports 1 (passed) or 0 (gave up); CTA `skip` never
@@ -821,224 +799,6 @@ __global__ void __launch_bounds__(KB) k_grid_barrier_check(unsigned int* count, 
     }
     const bool ok = grid_barrier(count, err, gridDim.x, max_polls);
     if (threadIdx.x == 0) result[blockIdx.x] = ok ? 1 : 0;
-}
-
-
-// The ELL words of one row held in registers for a whole launch (the
-// matrix does not change during a solve).
-template <int WW>
-struct SmallEll {
-    int32_t c[WW > 0 ? WW : 1];
-    double a[WW > 0 ? WW : 1];
-};
-
-template <int WW>
-__device__ __forceinline__ void small_load(const int32_t* __restrict__ cols, const double* __restrict__ vals,
-                                           int64_t rows, int64_t q, SmallEll<WW>& e)
-{
-#pragma unroll
-    for (int k = 0; k < WW; ++k) {
-        e.c[k] = __ldg(cols + (int64_t)k * rows + q);
-        e.a[k] = __ldg(vals + (int64_t)k * rows + q);
-    }
-}
-
-template <int WW, typename G>
-__device__ __forceinline__ double small_apply(const SmallEll<WW>& e, double self, G&& g)
-{
-    double xg[WW > 0 ? WW : 1];
-#pragma unroll
-    for (int k = 0; k < WW; ++k) xg[k] = g(e.c[k]);
-    double acc = self;
-#pragma unroll
-    for (int k = 0; k < WW; ++k) acc = fma(e.a[k], xg[k], acc);
-    return acc;
-}
-
-// Rows per thread whose ELL words stay in registers for the launch: two for
-// the compile-time widths up to 6, one for the wider ones, none for the
-// run-time width.
-constexpr int small_rows_in_registers(int WW) { return WW == 0 ? 0 : (WW <= 6 ? 2 : 1); }
-
-// Three phases and three grid barriers per iteration: the p update of the
-// previous iteration and the s update are formed where they are needed,
-// for the own rows and again for each gathered neighbour (the same
-// operations, so the same values), instead of in phases of their own.  p
-// and v therefore alternate between two buffers: the neighbours' old p and
-// v stay readable while the new ones are written.
-//  1. p = r + beta (p' - omega v') (on a restart and in the first
-//     iteration p = rh = r), v = A p, (rh, v) -> alpha;
-//  2. s = r - alpha v, t = A s, (t, s), (t, t), (s, s) -> the half-step
-//     test and omega;
-//  3. x += alpha p + omega s, r = s - omega t, (rh, r), (r, r) -> the
-//     convergence test, the restart test and beta.
-template <int WW>
-__global__ void __launch_bounds__(KB) k_bicgstab_small(const int32_t* __restrict__ cols,
-                                                       const double* __restrict__ vals, int W, int64_t rows,
-                                                       double* x, double* r, double* rh, double* p0, double* p1,
-                                                       double* v0, double* v1, double* s, double* t,
-                                                       KrylovScalars* sc, double* partials, unsigned int* bar,
-                                                       int* bar_err, int max_its)
-{
-    __shared__ KrylovScalars S;
-    if (threadIdx.x == 0) S = *sc;
-    __syncthreads();
-    if (S.done) return;
-    MHFEM_GRID_STRIDE;
-    const unsigned int nb = gridDim.x;
-    unsigned int target = 0;
-    double* pa = partials;
-    double* pc = partials + (int64_t)nb * kPartStride;
-    double* pd = partials + 2 * (int64_t)nb * kPartStride;
-    // The ELL words of the thread's first RK rows, loaded once: both SpMVs of
-    // every iteration then start with the gathers, one L2 round trip instead
-    // of two behind each grid barrier.
-    constexpr int RK = small_rows_in_registers(WW);
-    SmallEll<WW> er[RK > 0 ? RK : 1];
-#pragma unroll
-    for (int j = 0; j < RK; ++j) {
-        const int64_t q = gtid + (int64_t)j * gstride;
-        if (q < rows) small_load<WW>(cols, vals, rows, q, er[j]);
-    }
-    // For the widths up to 6, the own-row values of those rows that the
-    // third phase needs (p, rh, s, t, x) stay in registers from the phase
-    // that forms or loads them, so the third phase reaches its reduction
-    // without a memory round trip; s and t of these rows are then never
-    // stored.  (For the wider rows the extra registers cost more than the
-    // round trip: 36.1 against 35.2 us per iteration on the 128^2
-    // two-component system, width 9.)
-    constexpr int R3 = WW <= 6 ? RK : 0;
-    double preg[R3 > 0 ? R3 : 1], hreg[R3 > 0 ? R3 : 1], sreg[R3 > 0 ? R3 : 1], treg[R3 > 0 ? R3 : 1],
-        xreg[R3 > 0 ? R3 : 1];
-    // y = A x over the thread's rows with x given by xval (own row and
-    // gathered neighbours); the register rows first, all their loads ahead of
-    // their stores, then any further rows from the matrix in memory.
-    // finish(j, q, x_q, y_q) gets the register slot j, or -1.
-    auto spmv_rows = [&](auto&& xval, auto&& finish) {
-        double xr[RK > 0 ? RK : 1], yr[RK > 0 ? RK : 1];
-#pragma unroll
-        for (int j = 0; j < RK; ++j) {
-            const int64_t q = gtid + (int64_t)j * gstride;
-            if (q < rows) {
-                xr[j] = xval(q);
-                yr[j] = small_apply<WW>(er[j], xr[j], xval);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < RK; ++j) {
-            const int64_t q = gtid + (int64_t)j * gstride;
-            if (q < rows) finish(j, q, xr[j], yr[j]);
-        }
-        for (int64_t q = gtid + (int64_t)RK * gstride; q < rows; q += gstride) {
-            const double xq = xval(q);
-            finish(-1, q, xq, small_row<WW>(cols, vals, W, rows, q, xq, xval));
-        }
-    };
-    for (int k = 0; k < max_its; ++k) {
-        const int cur = S.it & 1;
-        const double* P = cur ? p1 : p0;
-        double* Pn = cur ? p0 : p1;
-        const double* V = cur ? v1 : v0;
-        double* Vn = cur ? v0 : v1;
-        // 1. p, v = A p, (rh, v) -> alpha
-        {
-            const bool fresh = S.restart || S.it == 0;
-            const double beta = S.beta, omega = S.omega;
-            auto pval = [&](int64_t j) {
-                const double rj = __ldcg(r + j);
-                return fresh ? rj : fma(beta, fma(-omega, __ldcg(V + j), __ldcg(P + j)), rj);
-            };
-            double acc[1] = {0};
-            spmv_rows(pval, [&](int j, int64_t q, double pq, double y) {
-                Pn[q] = pq;
-                Vn[q] = y;
-                double hq;
-                if (fresh) { hq = __ldcg(r + q); rh[q] = hq; }
-                else hq = rh[q];
-                acc[0] = fma(hq, y, acc[0]);
-                if (j >= 0 && j < R3) { preg[j] = pq; hreg[j] = hq; }
-            });
-            block_reduce_store<double, 1>(acc, pa);
-            if (!grid_barrier(bar, bar_err, target += nb)) return;
-            double sum[1];
-            grid_sums<1>(pa, sum);
-            if (threadIdx.x == 0) scalars_alpha(&S, sum);
-            __syncthreads();
-            if (S.done) break;
-        }
-        const double alpha = S.alpha;
-        // 2. s = r - alpha v, t = A s, (t, s), (t, t), (s, s) -> half step, omega
-        {
-            auto sval = [&](int64_t j) { return fma(-alpha, __ldcg(Vn + j), __ldcg(r + j)); };
-            double acc[3] = {0, 0, 0};
-            spmv_rows(sval, [&](int j, int64_t q, double sv, double y) {
-                if (j >= 0 && j < R3) {
-                    sreg[j] = sv;
-                    treg[j] = y;
-                    xreg[j] = x[q];  // own row, written only by this thread
-                }
-                else {
-                    s[q] = sv;
-                    t[q] = y;
-                }
-                acc[0] = fma(y, sv, acc[0]);
-                acc[1] = fma(y, y, acc[1]);
-                acc[2] = fma(sv, sv, acc[2]);
-            });
-            block_reduce_store<double, 3>(acc, pc);
-            if (!grid_barrier(bar, bar_err, target += nb)) return;
-            double sum[3];
-            grid_sums<3>(pc, sum);
-            if (threadIdx.x == 0) scalars_omega<true>(&S, sum);
-            __syncthreads();
-        }
-        if (S.half) {
-            for (int64_t q = gtid; q < rows; q += gstride) x[q] = fma(alpha, Pn[q], x[q]);
-            if (threadIdx.x == 0) scalars_half(&S);
-            __syncthreads();
-            break;
-        }
-        if (S.done) break;
-        // 3. x, r, (rh, r), (r, r) -> convergence, restart, beta
-        {
-            const double omega = S.omega;
-            double acc[2] = {0, 0};
-#pragma unroll
-            for (int j = 0; j < R3; ++j) {
-                const int64_t q = gtid + (int64_t)j * gstride;
-                if (q < rows) {
-                    const double sv = sreg[j];
-                    x[q] = fma(omega, sv, fma(alpha, preg[j], xreg[j]));
-                    const double rv = fma(-omega, treg[j], sv);
-                    r[q] = rv;
-                    acc[0] = fma(hreg[j], rv, acc[0]);
-                    acc[1] = fma(rv, rv, acc[1]);
-                }
-            }
-            for (int64_t q = gtid + (int64_t)R3 * gstride; q < rows; q += gstride) {
-                const double sv = s[q];
-                x[q] = fma(omega, sv, fma(alpha, Pn[q], x[q]));
-                const double rv = fma(-omega, t[q], sv);
-                r[q] = rv;
-                acc[0] = fma(rh[q], rv, acc[0]);
-                acc[1] = fma(rv, rv, acc[1]);
-            }
-            block_reduce_store<double, 2>(acc, pd);
-            if (!grid_barrier(bar, bar_err, target += nb)) return;
-            double sum[2];
-            grid_sums<2>(pd, sum);
-            if (threadIdx.x == 0) {
-                scalars_beta<true>(&S, sum);
-                if (!S.done && S.restart) {  // rh = r (formed in phase 1): rho = (r, r)
-                    S.rho = S.rr;
-                    S.rhnorm = sqrt(S.rr);
-                }
-            }
-            __syncthreads();
-            if (S.done) break;
-        }
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *sc = S;
 }
 
 // ---- launch shapes ---------------------------------------------------------------
@@ -1453,49 +1213,10 @@ void krylov_fp64_kernel_once(const EllMatrix& A, KrylovWork& W, int which, cudaS
 
 // ---- small systems: host side ----------------------------------------------------
 
-// Rows up to which the FP64 solve takes the persistent path, and rows per
-// thread it aims at (more CTAs spread the memory traffic over more SMs, but
-// every CTA adds an arrival to each grid barrier).
+// Rows up to which GMRES takes its persistent path (k_gmres_small).
 constexpr int64_t kSmallSystemRows = (int64_t)1 << 18;
-constexpr int kSmallRowsPerThread = 2;
 
 int64_t krylov_small_rows() { return kSmallSystemRows; }
-
-cudaError_t krylov_small_fp64(const EllMatrix& A, double* x, KrylovWork& W, int iters, cudaStream_t s)
-{
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    const int sms = sm_count(dev);
-    int nb = 0;
-    MHFEM_WIDTH_DISPATCH(A.width, e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_bicgstab_small<WW>, KB, 0));
-    if (e != cudaSuccess) return e;
-    if (nb < 1) return cudaErrorCooperativeLaunchTooLarge;
-    const int64_t want = (A.rows + (int64_t)KB * kSmallRowsPerThread - 1) / ((int64_t)KB * kSmallRowsPerThread);
-    // every CTA resident (a cooperative launch), at most one per SM, and few
-    // enough that the three reductions' partials fit the per-CTA buffer
-    int grid = (int)std::min<int64_t>(std::min<int64_t>(want, (int64_t)sms), (int64_t)nb * sms);
-    grid = std::max(1, std::min(grid, W.grid / 3));
-    unsigned int* bar = W.counters + 2;
-    int* bar_err = reinterpret_cast<int*>(W.counters + 3);
-    e = cudaMemsetAsync(bar, 0, 2 * sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
-    const int32_t* cols = A.cols;
-    const double* vals = A.vals;
-    int W_ = A.width;
-    int64_t rows = A.rows;
-    double *r = W.r, *rh = W.rh, *p0 = W.p, *p1 = W.p2, *v0 = W.v, *v1 = W.v2, *sv = W.s, *t = W.t;
-    if (!p1 || !v1) return cudaErrorInvalidValue;
-    KrylovScalars* sc = W.sc;
-    double* partials = W.partials;
-    int its = iters;
-    void* args[] = {(void*)&cols, (void*)&vals, (void*)&W_, (void*)&rows, (void*)&x, (void*)&r, (void*)&rh,
-                    (void*)&p0, (void*)&p1, (void*)&v0, (void*)&v1, (void*)&sv, (void*)&t, (void*)&sc,
-                    (void*)&partials, (void*)&bar, (void*)&bar_err, (void*)&its};
-    MHFEM_WIDTH_DISPATCH(A.width, e = cudaLaunchCooperativeKernel((const void*)k_bicgstab_small<WW>, dim3(grid), dim3(KB),
-                                                                 args, 0, s));
-    return e;
-}
 
 cudaError_t grid_barrier_check(int ctas, int skip, unsigned int max_polls, int* passed, int* gave_up, int* flag)
 {

@@ -9,10 +9,10 @@
 // right-hand side and the solution; this entry point borrows nothing else.
 //
 // The Krylov work vectors, the per-CTA partial sums and the device scalars
-// live in one file-scope static device array of fixed size (about 17 MB).
-// Every system it takes fits the persistent small-system solve (one
-// cooperative launch per chunk of 256 iterations, the convergence test in
-// every iteration), which mhfem_solve runs for the same sizes.
+// live in one file-scope static device array of fixed size (about 13 MB).
+// Every system it takes fits the resident solve (k_resident.cu: one launch
+// per chunk of 256 iterations, the convergence test in every iteration),
+// which mhfem_solve runs for the same sizes.
 // Under CUDA's lazy module loading the array is committed on a device at the
 // first call there (the cudaGetSymbolAddress below loads the module), not when
 // the library is loaded, and it stays until the process exits; systems with
@@ -27,12 +27,11 @@ namespace {
 
 constexpr int64_t kMaxRows = MHFEM_NOALLOC_MAX_ROWS;   // even: the vectors below are spaced by an even count
 constexpr int64_t kMaxGrid = 4096;                     // per-CTA partials (>= any Krylov grid here)
-constexpr int64_t kVecDoubles = 8 * kMaxRows;          // r, rh, p, v, s, t and the second p, v buffers
+constexpr int64_t kVecDoubles = 6 * kMaxRows;          // r, rh, p, v, s, t
 constexpr int64_t kPartialDoubles = 8 * kMaxGrid;
 constexpr int64_t kScalarDoubles = (sizeof(mhfem::KrylovScalars) + 7) / 8;
-// 8 uint32: [0] reduction ticket, [2] grid-barrier count and [3] its failure
-// flag (the small-system solve), [4] bad-column count
-constexpr int64_t kCounterDoubles = 4;
+// KrylovWork::counters ([4] is unused there: the bad-column count)
+constexpr int64_t kCounterDoubles = mhfem::kCounterWords / 2;
 constexpr int kBadColumns = 4;
 constexpr int64_t kScratchDoubles = kVecDoubles + kPartialDoubles + kScalarDoubles + kCounterDoubles;
 
@@ -114,8 +113,6 @@ extern "C" mhfem_status mhfem_bicgstab_noalloc(const int32_t* cols, const double
     W.v = base + 3 * ld;
     W.s = base + 4 * ld;
     W.t = base + 5 * ld;
-    W.p2 = base + 6 * ld;
-    W.v2 = base + 7 * ld;
     W.partials = base + kVecDoubles;
     W.sc = reinterpret_cast<mhfem::KrylovScalars*>(base + kVecDoubles + kPartialDoubles);
     W.counters = reinterpret_cast<uint32_t*>(base + kVecDoubles + kPartialDoubles + kScalarDoubles);
@@ -137,12 +134,12 @@ extern "C" mhfem_status mhfem_bicgstab_noalloc(const int32_t* cols, const double
     }
     mhfem::krylov_init_fp64(A, rhs, x, W, tol, max_iter, s);
     if (cudaGetLastError() != cudaSuccess) return MHFEM_ERR_CUDA;
-    bool small = rows <= mhfem::krylov_small_rows();  // always, at this size limit
+    bool resident = mhfem::krylov_resident_fits(rows, width);  // on a whole GPU always, at this size limit
     mhfem::KrylovScalars hs{};
     int32_t barrier_failed = 0;
     for (bool first = true;; first = false) {
         if (cudaMemcpyAsync(&hs, W.sc, sizeof(hs), cudaMemcpyDeviceToHost, s) != cudaSuccess) return MHFEM_ERR_CUDA;
-        if (small && cudaMemcpyAsync(&barrier_failed, W.counters + 3, sizeof(barrier_failed), cudaMemcpyDeviceToHost,
+        if (resident && cudaMemcpyAsync(&barrier_failed, W.counters + mhfem::kBarrierError, sizeof(barrier_failed), cudaMemcpyDeviceToHost,
                                      s) != cudaSuccess)
             return MHFEM_ERR_CUDA;
         if (cudaStreamSynchronize(s) != cudaSuccess) return MHFEM_ERR_CUDA;
@@ -154,18 +151,18 @@ extern "C" mhfem_status mhfem_bicgstab_noalloc(const int32_t* cols, const double
             if (residual) *residual = hs.res;
             return MHFEM_ERR_TIMEOUT;
         }
-        if (small) {
-            const cudaError_t e = mhfem::krylov_small_fp64(A, x, W, 256, s);
+        if (resident) {
+            const cudaError_t e = mhfem::krylov_resident_fp64(A, x, W, 256, s);
             if (first && e == cudaErrorCooperativeLaunchTooLarge) {
                 // the device cannot hold the grid at once (a partitioned or
                 // shared GPU): nothing ran, the five-kernel iteration goes on
                 cudaGetLastError();
-                small = false;
+                resident = false;
             }
             else if (e != cudaSuccess)
                 return MHFEM_ERR_CUDA;
         }
-        if (!small) mhfem::krylov_iterate_fp64(A, x, W, 8, s);
+        if (!resident) mhfem::krylov_iterate_fp64(A, x, W, 8, s);
         if (cudaGetLastError() != cudaSuccess) return MHFEM_ERR_CUDA;
     }
     if (iterations) *iterations = hs.it;

@@ -148,7 +148,6 @@ struct KrylovWork {
     int64_t rows = 0;
     int grid = 0, block = 256;
     double *r = nullptr, *rh = nullptr, *p = nullptr, *v = nullptr, *s = nullptr, *t = nullptr;
-    double *p2 = nullptr, *v2 = nullptr;  // second p and v buffers of the small-system solve
     float *r32 = nullptr, *rh32 = nullptr, *p32 = nullptr, *v32 = nullptr, *s32 = nullptr,
           *t32 = nullptr, *x32 = nullptr;
     double* partials = nullptr;      // [grid][8]
@@ -215,14 +214,25 @@ void gmres_update(double* x, GmresWork& G, int64_t rows, cudaStream_t s);
 cudaError_t gmres_small(const EllMatrix& A, const double* b, double* x, GmresWork& G, KrylovWork& W, bool reorth,
                         int iters, cudaStream_t s);
 void krylov_iterate_fp64(const EllMatrix& A, double* x, KrylovWork& W, int iters, cudaStream_t s);
-// Small systems (rows <= krylov_small_rows()): up to `iters` FP64 BiCGStab
-// iterations in one cooperative launch on a solve set up by krylov_init_fp64
-// (p and v alternate between W.p / W.p2 and W.v / W.v2); the two words at
-// W.counters + 2 are the grid barrier's arrival count and its failure flag
-// (non-zero after a barrier wait gave up).
+// Rows up to which GMRES takes its persistent path.
 int64_t krylov_small_rows();
-cudaError_t krylov_small_fp64(const EllMatrix& A, double* x, KrylovWork& W, int iters, cudaStream_t s);
-// One cooperative launch of `ctas` CTAs through the small-system solve's
+// Words of KrylovWork::counters: [0] the reductions' ticket, [2] and [3] the
+// grid barrier's arrival count and failure flag of the small-system GMRES ([3]
+// also the resident BiCGStab's flag), then the resident BiCGStab's four
+// arrival counters, each on a 128-byte line of its own.
+constexpr int kBarrierError = 3;
+constexpr int kBarrierFirst = 32;
+constexpr int kBarrierStride = 32;
+constexpr int kCounterWords = kBarrierFirst + 4 * kBarrierStride;
+// Whether a system of this size can run resident on the SMs of the current
+// device (k_resident.cu), and up to `iters` FP64 BiCGStab iterations of it in
+// one launch on a solve set up by krylov_init_fp64 (W.r, W.rh, W.p; W.v and
+// W.s are written).  The flag at W.counters + kBarrierError is non-zero after
+// a wait between its CTAs gave up.  cudaErrorCooperativeLaunchTooLarge: the
+// device cannot hold the launch at once, and nothing ran.
+bool krylov_resident_fits(int64_t rows, int width);
+cudaError_t krylov_resident_fp64(const EllMatrix& A, double* x, KrylovWork& W, int iters, cudaStream_t s);
+// One cooperative launch of `ctas` CTAs through the persistent solves'
 // bounded grid barrier, CTA `skip` (none if negative) never arriving; counts
 // the CTAs that passed and that gave up, and returns the failure flag.
 cudaError_t grid_barrier_check(int ctas, int skip, unsigned int max_polls, int* passed, int* gave_up, int* flag);
