@@ -12,6 +12,7 @@ import numpy as np
 import pytest
 
 from helpers import diffusion3d_n2, rel_err
+from mhfem import _lib as L
 from mhfem import problems
 from oracle.oracle import OracleModel
 
@@ -89,6 +90,34 @@ def test_resident_solve_continues_after_a_chunk(name, N):
     # two solutions with residuals of 1e-13 differ by at most 2e-13 times the
     # condition number, which is below 24 N^2 dt (heat) and 5e4 here
     assert rel_err(s.state()[0], m.Z_iF) < 1e-8
+    s.close()
+
+
+@pytest.mark.parametrize("name,N", [
+    ("heat2d", 6),            # one CTA
+    ("heat2d", 51),           # the largest cluster
+    ("heat2d", 53),           # the smallest grid
+    ("heat2d", 391),          # 459,425: the ELL words still in shared memory
+    ("heat2d", 405),          # 492,885: streamed
+    ("diffusion3d", 13),
+    ("diffusion3d", 33),      # 437,778: streamed
+    ("diffusion3d", 50),      # 1,515,000: x in shared memory, the largest width-6 system below
+    ("diffusion3d", 52),      # 1,703,520: five kernels
+    ("diffusion3d_box", 30),  # width 10
+    ("adr2d", 30),            # width 9
+])
+def test_resident_inner_solve_against_oracle(name, N):
+    """The mixed form, whose FP32 inner solve runs resident."""
+    p = _problem(name, N)
+    p.config.form = L.FORM_MIXED
+    s = problems.make_solver(p)
+    m = OracleModel.from_problem(p)
+    st = s.step(0.0, p.dt)
+    m.step(0.0, p.dt, 1e-13)
+    assert st["residual"] < 1e-13 and st["sweeps"] > 1
+    zf, zk = s.state()
+    assert rel_err(zf, m.Z_iF) < TOL_STATE
+    assert rel_err(zk, m.Z_iK) < TOL_STATE
     s.close()
 
 

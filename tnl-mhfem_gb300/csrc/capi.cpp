@@ -784,7 +784,7 @@ mhfem_status mhfem::run_fp64(mhfem_t h, double tol, int max_iter, int* iters, do
     if (h->opts.linear_solver == MHFEM_SOLVER_GMRES) return run_gmres(h, tol, max_iter, iters, res);
     const auto t0 = std::chrono::steady_clock::now();
     krylov_init_fp64(h->A, h->rhs, h->Z_iF, h->W, tol, max_iter, h->stream);
-    bool resident = krylov_resident_fits(h->A.rows, h->A.width);
+    bool resident = krylov_resident_fits(h->A.rows, h->A.width, false);
     if (resident) {
         // the system fits the SMs: chunks of iterations in one launch each
         // (k_resident.cu), one host round trip per chunk
@@ -846,10 +846,8 @@ mhfem_status mhfem::run_mixed(mhfem_t h, int* iters, int* sweeps, double* res)
     init.tol = h->opts.tol;
     init.max_iter = h->opts.max_sweeps;
     CK(cudaMemcpyAsync(h->W.sc, &init, sizeof(init), cudaMemcpyHostToDevice, h->stream));
-    if (!h->g32) {
-        mhfem_status st = build_graph(h, true, h->opts.check_every);
-        if (st) return st;
-    }
+    // the system fits the SMs: the inner iterations run resident (k_resident.cu)
+    bool resident = krylov_resident_fits(h->A.rows, h->A.width, true);
     int total_inner = 0;
     for (;;) {
         mixed_outer_residual(h->A, h->rhs, h->Z_iF, h->W, h->opts.tol, h->opts.max_sweeps, h->stream);
@@ -867,9 +865,32 @@ mhfem_status mhfem::run_mixed(mhfem_t h, int* iters, int* sweeps, double* res)
             return status_from_krylov(h, outer, "mixed-precision refinement");
         }
         while (!h->W.host_sc[1].done) {
-            CK(cudaGraphLaunch(h->g32, h->stream));
-            h->launches += 5 * h->g32_iters;
-            CK(cudaStreamSynchronize(h->stream));
+            if (resident) {
+                const cudaError_t e = krylov_resident_fp32(h->A, h->W, 256, h->stream);
+                if (e == cudaErrorCooperativeLaunchTooLarge) {
+                    // the device cannot hold the launch at once: nothing ran
+                    cudaGetLastError();
+                    resident = false;
+                    continue;
+                }
+                CK(e);
+                h->launches += 1;
+                CK(cudaMemcpyAsync(h->W.host_sc + 1, h->W.sc32, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, h->stream));
+                CK(cudaMemcpyAsync(h->host_err, h->W.counters + kBarrierError, sizeof(int32_t), cudaMemcpyDeviceToHost,
+                                   h->stream));
+                CK(cudaStreamSynchronize(h->stream));
+                if (*h->host_err)
+                    return fail(h, MHFEM_ERR_CUDA, "FP32 BiCGStab (resident): a grid barrier wait gave up");
+            }
+            else {
+                if (!h->g32) {
+                    mhfem_status st = build_graph(h, true, h->opts.check_every);
+                    if (st) return st;
+                }
+                CK(cudaGraphLaunch(h->g32, h->stream));
+                h->launches += 5 * h->g32_iters;
+                CK(cudaStreamSynchronize(h->stream));
+            }
             if (h->opts.timeout_s > 0 && elapsed_s(t0) > h->opts.timeout_s)
                 return fail(h, MHFEM_ERR_TIMEOUT, "mixed solve exceeded %.1f s", h->opts.timeout_s);
         }

@@ -134,7 +134,7 @@ extern "C" mhfem_status mhfem_bicgstab_noalloc(const int32_t* cols, const double
     }
     mhfem::krylov_init_fp64(A, rhs, x, W, tol, max_iter, s);
     if (cudaGetLastError() != cudaSuccess) return MHFEM_ERR_CUDA;
-    bool resident = mhfem::krylov_resident_fits(rows, width);  // on a whole GPU always, at this size limit
+    bool resident = mhfem::krylov_resident_fits(rows, width, false);  // on a whole GPU always, at this size limit
     mhfem::KrylovScalars hs{};
     int32_t barrier_failed = 0;
     for (bool first = true;; first = false) {

@@ -230,8 +230,10 @@ constexpr int kCounterWords = kBarrierFirst + 4 * kBarrierStride;
 // W.s are written).  The flag at W.counters + kBarrierError is non-zero after
 // a wait between its CTAs gave up.  cudaErrorCooperativeLaunchTooLarge: the
 // device cannot hold the launch at once, and nothing ran.
-bool krylov_resident_fits(int64_t rows, int width);
+bool krylov_resident_fits(int64_t rows, int width, bool fp32);
 cudaError_t krylov_resident_fp64(const EllMatrix& A, double* x, KrylovWork& W, int iters, cudaStream_t s);
+// The same for the mixed form's inner solve, set up by mixed_inner_init.
+cudaError_t krylov_resident_fp32(const EllMatrix& A, KrylovWork& W, int iters, cudaStream_t s);
 // One cooperative launch of `ctas` CTAs through the persistent solves'
 // bounded grid barrier, CTA `skip` (none if negative) never arriving; counts
 // the CTAs that passed and that gave up, and returns the failure flag.

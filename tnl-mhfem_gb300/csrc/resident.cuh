@@ -1,0 +1,694 @@
+#pragma once
+// BiCGStab with the system resident on the SMs (sm_103a): the FP64 solve
+// (k_resident.cu) and the mixed form's FP32 inner solve (k_resident32.cu).
+//
+// One launch runs a chunk of iterations.  Every CTA owns a contiguous block
+// of rows and keeps their Krylov vectors in shared memory for the whole
+// launch (for the smaller systems the rows' ELL words too), so that only
+// what the SpMVs gather goes through memory, and an iteration is three (or
+// four) phases separated by group-wide reductions instead of five kernels:
+//   A. v = A p, (rh, v) -> alpha;
+//   B. s = r - alpha v, t = A s, (t, s), (t, t), (rh, s), (rh, t) -> omega and
+//      beta;
+//   C. x += alpha p + omega s, r = s - omega t, p = r + beta (p - omega v),
+//      (r, r), (rh, r) -> the convergence and restart tests.
+// beta needs rho' = (rh, r) before r exists; it is taken from the sums of
+// phase B, (rh, s) - omega (rh, t), so that p is updated in the pass that
+// forms r.  The next alpha uses the rho' summed over r itself in phase C, so
+// the recurrence's rounding does not accumulate.
+//
+// What bounds it.  GB300 issues FP64 at 1.68 lanes per clock per SM (saturated
+// by four warps) with 64 cycles of latency, so a small system's iteration is a
+// chain of dependent FP64 additions, divisions and synchronisations: a warp
+// reduction takes 0.2 us, a division 0.27 us, a grid barrier 1.5 us.  Hence:
+//  - a reduction's sums go to different warps (one per FP64 unit of the SM),
+//    each with its own arrival counter, and no thread fence beyond the
+//    counter's own release and acquire;
+//  - the scalars take one reciprocal of three dependent operations per
+//    reduction, square roots only near the decisions they belong to;
+//  - the systems of a few thousand rows run in one thread-block cluster: its
+//    barrier takes 0.5 us and the gathers read the neighbours' shared memory.
+// Every wait on a grid counter is bounded: a CTA that polls kBarrierPolls
+// times records the failure in *bar_err and returns, and the others then fail
+// their waits too.
+#include <algorithm>
+#include <mutex>
+#include <set>
+#include <utility>
+
+#include "fp_convert.h"
+#include "krylov_common.cuh"
+
+namespace mhfem {
+
+namespace {
+
+constexpr int kMaxThreads = 512;
+constexpr int kSums = 4;          // sums of the widest reduction
+constexpr int kMaxCluster = 16;
+
+template <typename T>
+struct ResidentArgs {
+    const int32_t* cols;
+    const T* vals;
+    int W;
+    int64_t rows;
+    int rc;             // rows per CTA
+    int x_in_smem;
+    T *x, *r, *rh, *p, *v, *s;
+    KrylovScalars* sc;
+    double* partials;   // [3 reductions][kSums][CTA]
+    unsigned int* bar;  // kSums arrival counters, kBarrierStride words apart
+    int* bar_err;
+    int max_its;
+};
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// Address of the same shared variable in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank)
+{
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    return a;
+}
+template <typename T>
+__device__ __forceinline__ T ld_cluster(uint32_t addr)
+{
+    T v;
+    if constexpr (sizeof(T) == 8) asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
+    else asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_cluster(uint32_t addr, double v)
+{
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_barrier()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ double warp_sum(double v)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// A thread's sums enter the reductions as FP64 (converted off the FP64 pipe).
+__device__ __forceinline__ double widen(double v) { return v; }
+__device__ __forceinline__ double widen(float v) { return f32_to_f64(v); }
+
+// Sum of col[lane], col[lane + 32], ... over n values in four chains.
+__device__ __forceinline__ double lane_sum(const double* col, int lane, int n)
+{
+    double a[4] = {0, 0, 0, 0};
+    for (int j = lane; j < n; j += 128) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (j + 32 * k < n) a[k] = (j == lane) ? col[j + 32 * k] : a[k] + col[j + 32 * k];
+    }
+    return (a[0] + a[1]) + (a[2] + a[3]);
+}
+
+// The CTAs of the launch as one group: reductions over all of them and a
+// barrier.  CL: one cluster; else the whole (cooperatively launched) grid.
+template <bool CL>
+struct Group {
+    double* col;     // [kSums][threads]
+    double* tot;     // [kSums]
+    double* slots;   // cluster: [3][kSums][kMaxCluster]
+    int* bad;        // shared: a wait gave up
+    double* partials;
+    unsigned int* bar;
+    int* err;
+    unsigned int target = 0;  // arrivals this thread's counter (its warp's) has seen
+
+    // tot[q] = the sum of every thread's acc[q]; also a barrier that makes
+    // the global (or cluster-shared) writes before it visible after it.
+    // Reductions of different `kind` alternate, so a kind's buffer is free
+    // again when it is written next.
+    template <int NV, typename T_>
+    __device__ __forceinline__ bool reduce(const T_ (&acc)[NV], int kind)
+    {
+        const int T = blockDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nc = gridDim.x;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) col[q * T + threadIdx.x] = widen(acc[q]);
+        __syncthreads();
+        if constexpr (CL) {
+            double* mine = slots + (kind * kSums + warp) * kMaxCluster;
+            if (warp < NV) {
+                const double v = warp_sum(lane_sum(col + warp * T, lane, T));
+                if (lane < nc) st_cluster(map_rank(smem_u32(mine + blockIdx.x), lane), v);
+            }
+            cluster_barrier();
+            if (warp < NV) {
+                double v = lane < nc ? mine[lane] : 0.0;
+#pragma unroll
+                for (int o = kMaxCluster / 2; o > 0; o >>= 1)
+                    if (o < nc) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == 0) tot[warp] = v;
+            }
+            __syncthreads();
+            return true;
+        }
+        else {
+            if (warp < NV) {
+                double* mine = partials + (int64_t)(kind * kSums + warp) * nc;
+                const double v = warp_sum(lane_sum(col + warp * T, lane, T));
+                int ok = 1;
+                target += nc;
+                if (lane == 0) {
+                    __stcg(mine + blockIdx.x, v);
+                    ok = arrive_and_wait(bar + warp * kBarrierStride, err, target);
+                }
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                double a[5] = {0, 0, 0, 0, 0};  // at most one CTA per SM: 152 partials in one pass
+                if (ok)
+                    for (int b = lane; b < nc; b += 160) {
+                        double w[5];
+#pragma unroll
+                        for (int k = 0; k < 5; ++k) w[k] = b + 32 * k < nc ? __ldcg(mine + b + 32 * k) : 0.0;
+#pragma unroll
+                        for (int k = 0; k < 5; ++k) a[k] = b == lane ? w[k] : a[k] + w[k];
+                    }
+                const double s = warp_sum(((a[0] + a[1]) + (a[2] + a[3])) + a[4]);
+                if (lane == 0) {
+                    tot[warp] = s;
+                    if (!ok) *bad = 1;
+                }
+            }
+            __syncthreads();
+            return *bad == 0;
+        }
+    }
+
+    __device__ __forceinline__ bool barrier()
+    {
+        if constexpr (CL) {
+            cluster_barrier();
+            return true;
+        }
+        else {
+            __syncthreads();
+            if (threadIdx.x < 32) {
+                target += gridDim.x;
+                if (threadIdx.x == 0 && !arrive_and_wait(bar, err, target)) *bad = 1;
+            }
+            __syncthreads();
+            return *bad == 0;
+        }
+    }
+};
+
+// Tests on the bit pattern keep comparisons off the FP64 pipe (64 cycles each).
+__device__ __forceinline__ bool finite_bits(double v)
+{
+    return (__double_as_longlong(v) & 0x7ff0000000000000LL) != 0x7ff0000000000000LL;
+}
+__device__ __forceinline__ bool zero_bits(double v) { return (__double_as_longlong(v) << 1) == 0; }
+// a > b for a >= 0, b >= 0 and both finite
+__device__ __forceinline__ bool greater_bits(double a, double b)
+{
+    return __double_as_longlong(a) > __double_as_longlong(b);
+}
+
+constexpr double kTiny = 1e-280;  // squares above this are far from the range's end
+
+// Limits that decide a common iteration's end without a square root or a
+// quotient: (tol ||b||)^2 and (kRestartEps ||rh||)^2, each with a margin far
+// above the rounding of the comparison it stands for.
+struct EndLimits {
+    double conv2, restart2;
+};
+__device__ __forceinline__ EndLimits end_limits(const KrylovScalars& S)
+{
+    const double thr = S.tol * S.bnorm, e = kRestartEps * S.rhnorm;
+    return {thr * thr * (1.0 + 1e-12), e * e * (1.0 + 1e-9)};
+}
+
+// The decisions at the end of an iteration, as scalars_beta's (k_krylov.cu):
+// non-finite, converged, iteration cap, breakdown, restart.  S->res holds the
+// residual when the solve or the chunk ends.
+__device__ __forceinline__ void end_of_iteration(KrylovScalars* S, EndLimits* lim, double rr, double rho,
+                                                 bool last_of_chunk)
+{
+    const double rho2 = rho * rho, bound2 = lim->restart2 * rr;
+    S->it += 1;
+    S->rr = rr;
+    if (!last_of_chunk && S->it < S->max_iter && finite_bits(rr) && finite_bits(rho2) &&
+        greater_bits(lim->conv2, kTiny) && greater_bits(rr, lim->conv2) && greater_bits(bound2, kTiny) &&
+        greater_bits(rho2, bound2) && !zero_bits(S->omega) && !zero_bits(S->rho)) {
+        S->rho = rho;
+        S->restart = 0;
+        return;
+    }
+    S->res = sqrt(rr) / S->bnorm;
+    S->restart = 0;
+    if (!finite(S->res)) { S->status = KS_NOTFINITE; S->done = 1; }
+    else if (S->res < S->tol) { S->status = KS_CONVERGED; S->done = 1; }
+    else if (S->it >= S->max_iter) { S->status = KS_MAXITER; S->done = 1; }
+    else if (S->omega == 0 || S->rho == 0) { S->status = KS_BREAKDOWN; S->done = 1; }
+    else if (fabs(rho) <= kRestartEps * sqrt(rr) * S->rhnorm) {
+        // shadow residual (numerically) orthogonal to r: restart with rh = p = r
+        S->restart = 1;
+        S->rho = rr;
+        S->rhnorm = sqrt(rr);
+        *lim = end_limits(*S);
+    }
+    else
+        S->rho = rho;
+}
+
+// WW: compile-time ELL width (0: run-time).  MATS: the CTA's ELL words are
+// copied to shared memory once.  CL: one cluster, gathers from the CTAs'
+// shared memory.  RECOMP: phase B forms s at each gathered neighbour from its
+// r and v (W more FP64 operations per row) instead of publishing s behind a
+// barrier of its own.
+template <typename R, int WW, bool MATS, bool CL, bool RECOMP>
+__global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const ResidentArgs<R> g)
+{
+    static_assert(!CL || (MATS && RECOMP), "the cluster form keeps everything in shared memory");
+    extern __shared__ double smem[];
+    __shared__ KrylovScalars S;
+    __shared__ double tot[kSums];
+    __shared__ double s_inv_rv;
+    __shared__ double slots[CL ? 3 * kSums * kMaxCluster : 1];
+    __shared__ int bad;
+    const int T = blockDim.x, rc = g.rc, W = WW > 0 ? WW : g.W;
+    const int64_t base = (int64_t)blockIdx.x * rc, rows = g.rows;
+    const int n = (int)max((int64_t)0, min((int64_t)rc, rows - base));
+    __shared__ EndLimits limits;
+    if (threadIdx.x == 0) {
+        S = *g.sc;
+        limits = end_limits(S);
+        bad = 0;
+    }
+    __syncthreads();
+    if (S.done) return;  // the same in every CTA
+
+    double* col = smem;
+    R* sr = reinterpret_cast<R*>(col + kSums * T);
+    R* srh = sr + rc;
+    R* sp = srh + rc;
+    R* sv = sp + rc;
+    R* st = sv + rc;
+    R* ss = RECOMP ? st + rc : sr;  // without RECOMP s takes r's place
+    R* sa = st + (RECOMP ? 2 : 1) * rc;
+    R* xp = g.x + base;
+    if (g.x_in_smem) {
+        xp = sa;
+        sa += rc;
+    }
+    uint32_t* scol = reinterpret_cast<uint32_t*>(sa + (int64_t)(MATS ? W : 0) * rc);
+
+    for (int m = threadIdx.x; m < n; m += T) {
+        sr[m] = __ldcg(g.r + base + m);
+        srh[m] = __ldcg(g.rh + base + m);
+        sp[m] = __ldcg(g.p + base + m);
+        if (g.x_in_smem) xp[m] = g.x[base + m];
+    }
+    if constexpr (MATS)
+        for (int k = 0; k < W; ++k)
+            for (int m = threadIdx.x; m < n; m += T) {
+                const int64_t o = (int64_t)k * rows + base + m;
+                const uint32_t c = (uint32_t)__ldg(g.cols + o);
+                sa[k * rc + m] = __ldg(g.vals + o);
+                // cluster: the column's address in its owner's copy of sr
+                scol[k * rc + m] = CL ? map_rank(smem_u32(sr + c % rc), c / rc) : c;
+            }
+    Group<CL> G{col, tot, slots, &bad, g.partials, g.bar, g.bar_err};
+    if constexpr (CL) cluster_barrier();  // every CTA's shared memory is set up
+    else __syncthreads();
+
+    // y = self + sum_k a_k gather(c_k) over the CTA's rows; body(m, y).  The
+    // streamed form loads the next row's ELL words before the current gathers.
+    auto spmv = [&](auto&& self, auto&& gather, auto&& body) {
+        if constexpr (MATS) {
+            for (int m = threadIdx.x; m < n; m += T) {
+                R y = self(m);
+                if constexpr (WW > 0) {
+                    R xg[WW];
+#pragma unroll
+                    for (int k = 0; k < WW; ++k) xg[k] = gather(scol[k * rc + m]);
+#pragma unroll
+                    for (int k = 0; k < WW; ++k) y = fma(sa[k * rc + m], xg[k], y);
+                }
+                else {
+                    for (int k = 0; k < W; ++k) y = fma(sa[k * rc + m], gather(scol[k * rc + m]), y);
+                }
+                body(m, y);
+            }
+        }
+        else if constexpr (WW > 0 && WW <= 6) {
+            int32_t c[WW];
+            R a[WW];
+            auto load = [&](int m, int32_t(&cc)[WW], R(&aa)[WW]) {
+#pragma unroll
+                for (int k = 0; k < WW; ++k) {
+                    cc[k] = __ldg(g.cols + (int64_t)k * rows + base + m);
+                    aa[k] = __ldg(g.vals + (int64_t)k * rows + base + m);
+                }
+            };
+            int m = threadIdx.x;
+            if (m < n) load(m, c, a);
+            for (; m < n; m += T) {
+                int32_t cn[WW];
+                R an[WW];
+                if (m + T < n) load(m + T, cn, an);
+                R xg[WW];
+#pragma unroll
+                for (int k = 0; k < WW; ++k) xg[k] = gather((uint32_t)c[k]);
+                R y = self(m);
+#pragma unroll
+                for (int k = 0; k < WW; ++k) y = fma(a[k], xg[k], y);
+                body(m, y);
+#pragma unroll
+                for (int k = 0; k < WW; ++k) {
+                    c[k] = cn[k];
+                    a[k] = an[k];
+                }
+            }
+        }
+        else {
+            for (int m = threadIdx.x; m < n; m += T) {
+                R y = self(m);
+                if constexpr (WW > 0) {
+                    int32_t c[WW];
+                    R a[WW], xg[WW];
+#pragma unroll
+                    for (int k = 0; k < WW; ++k) {
+                        c[k] = __ldg(g.cols + (int64_t)k * rows + base + m);
+                        a[k] = __ldg(g.vals + (int64_t)k * rows + base + m);
+                    }
+#pragma unroll
+                    for (int k = 0; k < WW; ++k) xg[k] = gather((uint32_t)c[k]);
+#pragma unroll
+                    for (int k = 0; k < WW; ++k) y = fma(a[k], xg[k], y);
+                }
+                else {
+                    for (int k = 0; k < W; ++k) {
+                        const int64_t o = (int64_t)k * rows + base + m;
+                        y = fma(__ldg(g.vals + o), gather((uint32_t)__ldg(g.cols + o)), y);
+                    }
+                }
+                body(m, y);
+            }
+        }
+    };
+    const uint32_t off_p = (uint32_t)((char*)sp - (char*)sr), off_v = (uint32_t)((char*)sv - (char*)sr);
+
+    for (int k = 0; k < g.max_its; ++k) {
+        // A. v = A p, (rh, v) -> alpha
+        {
+            R acc[1] = {0};
+            spmv([&](int m) { return sp[m]; },
+                 [&](uint32_t c) { return CL ? ld_cluster<R>(c + off_p) : g.p[c]; },
+                 [&](int m, R y) {
+                     sv[m] = y;
+                     if (RECOMP && !CL) __stcg(g.v + base + m, y);
+                     acc[0] = fma(srh[m], y, acc[0]);
+                 });
+            if (!G.reduce(acc, 0)) return;
+            if (threadIdx.x == 0) {
+                const double rv = tot[0], inv = recip_newton(rv);
+                S.rv = rv;
+                S.alpha = S.rho * inv;
+                s_inv_rv = inv;
+                if (!finite_bits(rv) || zero_bits(rv)) {
+                    S.status = finite_bits(rv) ? KS_BREAKDOWN : KS_NOTFINITE;
+                    S.done = 1;
+                    S.res = sqrt(S.rr) / S.bnorm;
+                }
+            }
+            __syncthreads();
+            if (S.done) break;
+        }
+        const R alpha = (R)S.alpha;
+        // B. s, t = A s, the four sums -> omega, beta
+        {
+            R acc[4] = {0, 0, 0, 0};
+            auto dots = [&](int m, R sv_, R y) {
+                const R h = srh[m];
+                acc[0] = fma(y, sv_, acc[0]);
+                acc[1] = fma(y, y, acc[1]);
+                acc[2] = fma(h, sv_, acc[2]);
+                acc[3] = fma(h, y, acc[3]);
+            };
+            if constexpr (RECOMP) {
+                spmv([&](int m) { return ss[m] = fma(-alpha, sv[m], sr[m]); },
+                     [&](uint32_t c) {
+                         return CL ? fma(-alpha, ld_cluster<R>(c + off_v), ld_cluster<R>(c))
+                                   : fma(-alpha, g.v[c], g.r[c]);
+                     },
+                     [&](int m, R y) {
+                         st[m] = y;
+                         dots(m, ss[m], y);
+                     });
+            }
+            else {
+                for (int m = threadIdx.x; m < n; m += T) {
+                    const R sv_ = fma(-alpha, sv[m], sr[m]);
+                    ss[m] = sv_;
+                    __stcg(g.s + base + m, sv_);
+                }
+                if (!G.barrier()) return;
+                spmv([&](int m) { return ss[m]; }, [&](uint32_t c) { return g.s[c]; },
+                     [&](int m, R y) {
+                         st[m] = y;
+                         dots(m, ss[m], y);
+                     });
+            }
+            if (!G.reduce(acc, 1)) return;
+            if (threadIdx.x < 2) {  // two quotients in two lanes: omega = ts / tt, then beta from tt / ts
+                const double ts = tot[0], tt = tot[1];
+                const double num = threadIdx.x == 0 ? ts : tt, den = threadIdx.x == 0 ? tt : ts;
+                const double q = num * recip_newton(den);
+                if (threadIdx.x == 0) {
+                    S.ts = ts;
+                    S.tt = tt;
+                    S.omega = q;
+                    S.half = 0;
+                    if (!finite_bits(ts) || !finite_bits(tt)) {
+                        S.status = KS_NOTFINITE;
+                        S.done = 1;
+                        S.res = sqrt(S.rr) / S.bnorm;
+                    }
+                    // A s = 0 with a nonsingular matrix: s = 0, and x + alpha p solves the system
+                    else if (zero_bits(tt)) S.half = 1;
+                }
+                else
+                    // beta = (rho' / rho) (alpha / omega) with alpha = rho / (rh, v) and
+                    // rho' = (rh, s) - omega (rh, t)
+                    S.beta = fma(tot[2], q, -tot[3]) * s_inv_rv;
+            }
+            __syncthreads();
+            if (S.done) break;
+        }
+        if (S.half) {
+            for (int m = threadIdx.x; m < n; m += T) xp[m] = fma(alpha, sp[m], xp[m]);
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                S.snorm = 0;
+                S.res = 0;
+                S.it += 1;
+                S.status = KS_CONVERGED;
+                S.done = 1;
+            }
+            __syncthreads();
+            break;
+        }
+        // C. x, r, p, (r, r), (rh, r) -> convergence, restart
+        {
+            const R omega = (R)S.omega, beta = (R)S.beta;
+            R acc[2] = {0, 0};
+            for (int m = threadIdx.x; m < n; m += T) {
+                const R sv_ = ss[m], pv = sp[m];
+                xp[m] = fma(omega, sv_, fma(alpha, pv, xp[m]));
+                const R rv = fma(-omega, st[m], sv_);
+                const R pn = fma(beta, fma(-omega, sv[m], pv), rv);
+                sr[m] = rv;
+                sp[m] = pn;
+                if (!CL) {
+                    __stcg(g.p + base + m, pn);
+                    if (RECOMP) __stcg(g.r + base + m, rv);
+                }
+                acc[0] = fma(rv, rv, acc[0]);
+                acc[1] = fma(srh[m], rv, acc[1]);
+            }
+            if (!G.reduce(acc, 2)) return;
+            if (threadIdx.x == 0) end_of_iteration(&S, &limits, tot[0], tot[1], k + 1 == g.max_its);
+            __syncthreads();
+            if (S.done) break;
+            if (S.restart) {
+                for (int m = threadIdx.x; m < n; m += T) {
+                    const R rv = sr[m];
+                    srh[m] = rv;
+                    sp[m] = rv;
+                    if (!CL) __stcg(g.p + base + m, rv);
+                }
+                if (!G.barrier()) return;
+            }
+        }
+    }
+    for (int m = threadIdx.x; m < n; m += T) {
+        if (g.x_in_smem) g.x[base + m] = xp[m];
+        g.r[base + m] = sr[m];
+        g.rh[base + m] = srh[m];
+        g.p[base + m] = sp[m];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *g.sc = S;
+    if constexpr (CL) cluster_barrier();  // no CTA leaves while another may still read its shared memory
+}
+
+// ---- launch shapes ---------------------------------------------------------------
+
+// Rows up to which one cluster takes the system.
+constexpr int64_t kClusterRows = 8192;
+// Off-diagonal entries up to which phase B of the FP64 solve forms the
+// neighbours' s itself: a barrier less against one FP64 operation per entry.
+// Measured per iteration, with and without: 14.97 and 15.84 us at 0.30M
+// entries (50,688 rows, width 6), 18.5 and 19.0 at 0.68M, 20.6 and 21.0 at
+// 0.79M (width 4), but 22.3 and 21.4 at 1.22M (width 9), 27.1 and 26.4 at
+// 1.44M.  In FP32 the operation costs nothing: always.
+constexpr int64_t kRecompEntries = 1000000;
+
+// Matrix bytes up to which the ELL words are streamed from L2 by one CTA per
+// SM (129 MB of L2 also holds the gathered vectors and x).  Measured per
+// iteration against the five kernels: 48.7 and 57.3 us at 44 MB (width 6),
+// 55.0 and 64.6 at 56 MB, 45.9 and 64.7 at 64 MB (width 10), but 77.0 and
+// 72.9 at 84 MB (width 9), 80.4 and 76.0 at 87 MB (width 10).
+// In FP32 (with half the vectors' bytes) 42.8 and 56.4 us at 73 MB.
+constexpr int64_t kStreamedBytes = (int64_t)72 << 20;
+
+struct ResidentPlan {
+    bool ok = false, cluster = false, mats = false, recomp = false, x_in_smem = false;
+    int ctas = 0, threads = 0, rc = 0;
+    size_t smem = 0;
+};
+
+ResidentPlan plan_resident(int64_t rows, int width, size_t real, int sms, size_t smem_max)
+{
+    ResidentPlan P;
+    if (rows < 1) return P;
+    auto fill = [&](int ctas) {
+        P.ctas = ctas;
+        P.rc = (int)((rows + ctas - 1) / ctas);
+        P.ctas = (int)((rows + P.rc - 1) / P.rc);  // no empty CTA
+        P.threads = P.rc <= 128 ? 128 : (P.rc <= 512 ? 256 : kMaxThreads);
+        const size_t vectors = 5 + (P.recomp ? 1 : 0) + (P.x_in_smem ? 1 : 0);
+        P.smem = sizeof(double) * (size_t)kSums * P.threads + real * vectors * P.rc +
+                 (P.mats ? (real + sizeof(int32_t)) * (size_t)width * P.rc : 0);
+        return P.smem + 2048 <= smem_max;  // 2 KB for the static shared variables
+    };
+    if (rows <= kClusterRows) {
+        int c = 1;
+        while (c < kMaxCluster && (int64_t)c * 128 < rows) c *= 2;
+        P.cluster = P.mats = P.recomp = P.x_in_smem = true;
+        // every CTA of the cluster is launched, also those left without rows
+        P.ok = fill(c);
+        P.ctas = c;
+        if (P.ok) return P;
+    }
+    const int64_t want = (rows + 127) / 128;
+    const int ctas = (int)std::min<int64_t>(want, sms);
+    for (int form = 0; form < 3; ++form) {  // ELL words and x in shared memory, x only, neither
+        if (form > 0 && (int64_t)(real + 4) * width * rows > kStreamedBytes) return ResidentPlan{};
+        P = ResidentPlan{};
+        P.mats = form == 0;
+        P.recomp = P.mats && (real == 4 || rows * width <= kRecompEntries);
+        P.x_in_smem = form < 2;
+        P.ok = fill(ctas);
+        if (P.ok) return P;
+    }
+    return P;
+}
+
+template <typename R, int WW, bool MATS, bool CL, bool RECOMP>
+cudaError_t launch_resident(const ResidentPlan& P, const ResidentArgs<R>& a, int dev, cudaStream_t s)
+{
+    auto kernel = k_bicgstab_resident<R, WW, MATS, CL, RECOMP>;
+    {
+        static std::mutex mu;
+        static std::set<int> done;  // devices on which the kernel's attributes are set
+        std::lock_guard<std::mutex> lock(mu);
+        if (!done.count(dev)) {
+            int most = 0;
+            cudaError_t e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+            cudaFuncAttributes fa{};
+            if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, kernel);
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         most - (int)fa.sharedSizeBytes);
+            if (CL && e == cudaSuccess)
+                e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            if (e != cudaSuccess) return e;
+            done.insert(dev);
+        }
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(P.ctas);
+    cfg.blockDim = dim3(P.threads);
+    cfg.dynamicSmemBytes = P.smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    if (CL) {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = P.ctas;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+    }
+    else {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a);
+    // a device (or partition of one) without room for the cluster refuses it
+    // as the cooperative launch does
+    return e == cudaErrorInvalidClusterSize ? cudaErrorCooperativeLaunchTooLarge : e;
+}
+
+template <typename R, int WW>
+cudaError_t launch_form(const ResidentPlan& P, const ResidentArgs<R>& a, int dev, cudaStream_t s)
+{
+    if (P.cluster) return launch_resident<R, WW, true, true, true>(P, a, dev, s);
+    if (P.mats && P.recomp) return launch_resident<R, WW, true, false, true>(P, a, dev, s);
+    if constexpr (sizeof(R) == 8)
+        if (P.mats) return launch_resident<R, WW, true, false, false>(P, a, dev, s);
+    return launch_resident<R, WW, false, false, false>(P, a, dev, s);
+}
+
+cudaError_t device_plan(int64_t rows, int width, size_t real, int* dev, ResidentPlan* P)
+{
+    cudaError_t e = cudaGetDevice(dev);
+    if (e != cudaSuccess) return e;
+    int most = 0;
+    e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, *dev);
+    if (e != cudaSuccess) return e;
+    *P = plan_resident(rows, width, real, sm_count(*dev), (size_t)most);
+    return cudaSuccess;
+}
+
+template <typename R>
+cudaError_t iterate_resident(const EllMatrix& A, const R* vals, R* x, R* r, R* rh, R* p, R* v, R* sv, KrylovScalars* sc,
+                             KrylovWork& W, int iters, cudaStream_t s)
+{
+    int dev = 0;
+    ResidentPlan P;
+    cudaError_t e = device_plan(A.rows, A.width, sizeof(R), &dev, &P);
+    if (e != cudaSuccess) return e;
+    if (!P.ok || (int64_t)3 * kSums * P.ctas > (int64_t)W.grid * kPartStride) return cudaErrorCooperativeLaunchTooLarge;
+    e = cudaMemsetAsync(W.counters, 0, kCounterWords * sizeof(uint32_t), s);
+    if (e != cudaSuccess) return e;
+    const ResidentArgs<R> a{A.cols, vals, A.width, A.rows, P.rc, P.x_in_smem ? 1 : 0, x, r, rh, p, v, sv, sc, W.partials,
+                            W.counters + kBarrierFirst, reinterpret_cast<int*>(W.counters + kBarrierError), iters};
+    MHFEM_WIDTH_DISPATCH(A.width, e = (launch_form<R, WW>(P, a, dev, s)));
+    return e;
+}
+
+}  // namespace
+
+}  // namespace mhfem
