@@ -347,8 +347,8 @@ mhfem_status mhfem_get_stream(mhfem_t h, void** stream);
 mhfem_status mhfem_time_kernel(mhfem_t h, int32_t kernel, int32_t reps, double* ms_per_launch,
                                double* bytes_per_launch, double* flops_per_launch);
 
-/* Check of the bounded grid barrier that the persistent solves (the resident
- * FP64 BiCGStab, the GMRES of at most 2^18 rows) place between their phases.  One cooperative launch of `ctas` CTAs on `device`
+/* Check of the bounded grid barrier that the resident solves (BiCGStab and
+ * GMRES of systems that fit the SMs) place between their phases.  One cooperative launch of `ctas` CTAs on `device`
  * passes through the barrier once, every wait polling at most `max_polls`
  * times; CTA `skip_cta` (none if negative) never arrives, so the others'
  * waits run out, set the failure flag and return -- the kernel ends without

@@ -121,6 +121,35 @@ def test_resident_inner_solve_against_oracle(name, N):
     s.close()
 
 
+@pytest.mark.parametrize("variant", ["cgs", "cgsr"])
+@pytest.mark.parametrize("name,N", [
+    ("heat2d", 2),             # one CTA, the Krylov space as large as the system
+    ("heat2d", 17),            # a cluster, the last block partial
+    ("heat2d", 51),            # the largest cluster
+    ("heat2d", 53),            # the smallest grid
+    ("heat2d", 150),           # 67,800: the basis in shared memory
+    ("heat2d", 200),           # 120,400: the basis in memory
+    ("heat2d", 300),           # 270,600
+    ("diffusion3d", 6),        # width 6
+    ("adr2d", 40),             # width 9
+    ("diffusion3d_box", 12),   # width 10
+    ("diffusion3d_n2", 5),     # width 13
+])
+def test_resident_gmres_against_oracle(name, N, variant):
+    p = _problem(name, N)
+    s = problems.make_solver(p)
+    s.setup(tol=1e-13, max_iter=20000, linear_solver="gmres", gmres_restart=30, gmres_variant=variant,
+            gmres_restart_min=3, gmres_restart_step_min=2, gmres_restart_step_max=4)
+    m = OracleModel.from_problem(p)
+    st = s.step(0.0, p.dt)
+    m.step(0.0, p.dt, 1e-13)
+    assert st["residual"] < 1e-13
+    zf, zk = s.state()
+    assert rel_err(zf, m.Z_iF) < TOL_STATE
+    assert rel_err(zk, m.Z_iK) < TOL_STATE
+    s.close()
+
+
 def test_resident_solve_iteration_cap():
     p = _problem("heat2d", 64)
     s = problems.make_solver(p, max_iter=7)

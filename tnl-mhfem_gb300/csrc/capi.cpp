@@ -703,14 +703,14 @@ mhfem_status run_gmres(mhfem_t h, double tol, int max_iter, int* iters, double* 
     double res_prev = G.host->res;
     const bool reorth = h->opts.gmres_variant == MHFEM_GMRES_CGSR;
     if (rows <= krylov_small_rows() && !G.host->done) {
-        // small system: chunks of iterations, restarts included, in one
-        // persistent launch each (k_gmres_small), one host round trip per
-        // chunk; the device applies the restart rule
+        // the system fits: chunks of iterations, restarts included, in one
+        // launch each (k_gmres_resident.cu), one host round trip per chunk;
+        // the device applies the restart rule
         CK(cudaMemcpyAsync(&G.st->res_prev, &res_prev, sizeof(double), cudaMemcpyHostToDevice, h->stream));
         constexpr int kChunk = 256;
         bool small = true;
         for (bool first = true;; first = false) {
-            const cudaError_t e = gmres_small(h->A, h->rhs, h->Z_iF, G, h->W, reorth, kChunk, h->stream);
+            const cudaError_t e = gmres_resident(h->A, h->rhs, h->Z_iF, G, h->W, reorth, kChunk, h->stream);
             if (first && e == cudaErrorCooperativeLaunchTooLarge) {
                 // the device cannot hold the grid at once: nothing ran, the
                 // graph of iterations below goes on from the same state
@@ -721,9 +721,9 @@ mhfem_status run_gmres(mhfem_t h, double tol, int max_iter, int* iters, double* 
             CK(e);
             h->launches += 1;
             CK(cudaMemcpyAsync(G.host, &G.st->ctl, sizeof(GmresCtl), cudaMemcpyDeviceToHost, h->stream));
-            CK(cudaMemcpyAsync(h->host_err, h->W.counters + 3, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+            CK(cudaMemcpyAsync(h->host_err, h->W.counters + kBarrierError, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
             CK(cudaStreamSynchronize(h->stream));
-            if (*h->host_err) return fail(h, MHFEM_ERR_CUDA, "GMRES (small system): a grid barrier wait gave up");
+            if (*h->host_err) return fail(h, MHFEM_ERR_CUDA, "GMRES (resident): a grid barrier wait gave up");
             if (G.host->done) break;
             if (h->opts.timeout_s > 0 && elapsed_s(t0) > h->opts.timeout_s)
                 return fail(h, MHFEM_ERR_TIMEOUT, "Krylov solve exceeded %.1f s", h->opts.timeout_s);
@@ -803,7 +803,7 @@ mhfem_status mhfem::run_fp64(mhfem_t h, double tol, int max_iter, int* iters, do
             CK(e);
             h->launches += 1;
             CK(cudaMemcpyAsync(h->W.host_sc, h->W.sc, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, h->stream));
-            CK(cudaMemcpyAsync(h->host_err, h->W.counters + 3, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+            CK(cudaMemcpyAsync(h->host_err, h->W.counters + kBarrierError, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
             CK(cudaStreamSynchronize(h->stream));
             if (*h->host_err)
                 return fail(h, MHFEM_ERR_CUDA, "FP64 BiCGStab (resident): a grid barrier wait gave up");

@@ -10,7 +10,7 @@
 // parameter in GMRES(m)", J. Comput. Appl. Math. 230 (2009) 751-761).  With
 // cr = ||r_j|| / ||r_{j-1}||, the ratio of the true residual norms at two
 // consecutive restarts (applied between cycles by the host, or inside the
-// persistent small-system solve by the device: next_restart_with):
+// resident solve by the device: next_restart_with):
 //  - cr > cos(8 deg) (the last cycle stagnated): m = m_max;
 //  - cr < cos(80 deg) (it converged well): m stays;
 //  - otherwise m decreases by the step d, and wraps to m_max when it would

@@ -320,8 +320,7 @@ __device__ __forceinline__ void stv(T* p, int64_t q, const VecT<T, V>& x)
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-// ---- persistent solves: bounded grid barriers (k_resident.cu, k_gmres_small), sums
-// in CTA order and gathered SpMV rows (k_gmres_small) ------------------------------
+// ---- bounded grid barriers of the resident solves (resident.cuh) ------------------
 //
 // Every barrier wait is bounded: a CTA that polls kBarrierPolls times
 // records the failure in *bar_err and returns, and the others then fail
@@ -367,64 +366,6 @@ __device__ __forceinline__ bool grid_barrier(unsigned int* count, int* err, unsi
     if (threadIdx.x == 0) ok = arrive_and_wait(count, err, target, max_polls) ? 1 : 0;
     __syncthreads();
     return ok != 0;
-}
-
-// Sum of the per-CTA partials [cta][kPartStride] in CTA order, identical in
-// every CTA (same loads, same order); the result is in out[] of every thread.
-template <int NV>
-__device__ __forceinline__ void grid_sums(const double* partials, double (&out)[NV])
-{
-    __shared__ double col[NV][KB];
-    __shared__ double tot[NV];
-    const int nb = (int)gridDim.x;
-#pragma unroll
-    for (int q = 0; q < NV; ++q)
-        col[q][threadIdx.x] = threadIdx.x < nb ? __ldcg(partials + (int64_t)threadIdx.x * kPartStride + q) : 0.0;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-#pragma unroll
-        for (int q = 0; q < NV; ++q) {
-            double v = col[q][lane];
-#pragma unroll
-            for (int w = 1; w < KB / 32; ++w) v += col[q][lane + 32 * w];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if (lane == 0) tot[q] = v;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < NV; ++q) out[q] = tot[q];
-}
-
-// y = self + sum_k a_k g(c_k), where g(j) forms the gathered vector's value
-// at row j (loaded past L1); same operation order as spmv_rows, so the
-// products match the five-kernel path's.
-template <int WW, typename G>
-__device__ __forceinline__ double small_row(const int32_t* __restrict__ cols, const double* __restrict__ vals, int W,
-                                            int64_t rows, int64_t q, double self, G&& g)
-{
-    double acc = self;
-    if constexpr (WW > 0) {
-        int32_t c[WW];
-        double a[WW], xg[WW];
-#pragma unroll
-        for (int k = 0; k < WW; ++k) {
-            c[k] = __ldg(cols + (int64_t)k * rows + q);
-            a[k] = __ldg(vals + (int64_t)k * rows + q);
-        }
-#pragma unroll
-        for (int k = 0; k < WW; ++k) xg[k] = g(c[k]);
-#pragma unroll
-        for (int k = 0; k < WW; ++k) acc = fma(a[k], xg[k], acc);
-    }
-    else
-        for (int k = 0; k < W; ++k) {
-            const int64_t o = (int64_t)k * rows + q;
-            acc = fma(__ldg(vals + o), g(__ldg(cols + o)), acc);
-        }
-    return acc;
 }
 
 }  // namespace mhfem

@@ -184,7 +184,7 @@ struct GmresState {
     double H[kGmresMaxM + 1][kGmresMaxM];
     double cs[kGmresMaxM], sn[kGmresMaxM];
     double g[kGmresMaxM + 1];
-    // restarts inside the persistent small-system solve: the true relative
+    // restarts inside the resident solve: the true relative
     // residual at the last restart, and the adaptive restart rule
     // (gmres_restart.h) with its two thresholds
     double res_prev;
@@ -209,17 +209,16 @@ void gmres_iterate(const EllMatrix& A, GmresWork& G, KrylovWork& W, int iters, b
 // end of a cycle: solve the triangular system and update x
 void gmres_update(double* x, GmresWork& G, int64_t rows, cudaStream_t s);
 // Small systems (at most krylov_small_rows() rows): up to `iters` Arnoldi
-// iterations, restarts included, in one cooperative launch (bounded grid
-// barriers; W.counters + 2 and + 3 are its barrier count and failure flag).
-cudaError_t gmres_small(const EllMatrix& A, const double* b, double* x, GmresWork& G, KrylovWork& W, bool reorth,
-                        int iters, cudaStream_t s);
+// iterations, restarts included, in one launch (k_gmres_resident.cu; the flag
+// at W.counters + kBarrierError as for krylov_resident_fp64).
+cudaError_t gmres_resident(const EllMatrix& A, const double* b, double* x, GmresWork& G, KrylovWork& W, bool reorth,
+                           int iters, cudaStream_t s);
 void krylov_iterate_fp64(const EllMatrix& A, double* x, KrylovWork& W, int iters, cudaStream_t s);
-// Rows up to which GMRES takes its persistent path.
+// Rows up to which GMRES runs resident.
 int64_t krylov_small_rows();
-// Words of KrylovWork::counters: [0] the reductions' ticket, [2] and [3] the
-// grid barrier's arrival count and failure flag of the small-system GMRES ([3]
-// also the resident BiCGStab's flag), then the resident BiCGStab's four
-// arrival counters, each on a 128-byte line of its own.
+// Words of KrylovWork::counters: [0] the reductions' ticket, [3] the flag of a
+// resident solve's wait that gave up, then the resident solves' four arrival
+// counters, each on a 128-byte line of its own.
 constexpr int kBarrierError = 3;
 constexpr int kBarrierFirst = 32;
 constexpr int kBarrierStride = 32;

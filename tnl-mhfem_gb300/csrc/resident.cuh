@@ -84,9 +84,12 @@ __device__ __forceinline__ void st_cluster(uint32_t addr, double v)
 {
     asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
 }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_barrier()
 {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_arrive();
+    cluster_wait();
 }
 
 __device__ __forceinline__ double warp_sum(double v)
@@ -128,9 +131,15 @@ struct Group {
     // tot[q] = the sum of every thread's acc[q]; also a barrier that makes
     // the global (or cluster-shared) writes before it visible after it.
     // Reductions of different `kind` alternate, so a kind's buffer is free
-    // again when it is written next.
+    // again when it is written next.  The warps that have no sum to take run
+    // side() while the others wait.
     template <int NV, typename T_>
     __device__ __forceinline__ bool reduce(const T_ (&acc)[NV], int kind)
+    {
+        return reduce<NV>(acc, kind, [](int) {});
+    }
+    template <int NV, typename T_, typename Side>
+    __device__ __forceinline__ bool reduce(const T_ (&acc)[NV], int kind, Side&& side)
     {
         const int T = blockDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nc = gridDim.x;
 #pragma unroll
@@ -142,7 +151,9 @@ struct Group {
                 const double v = warp_sum(lane_sum(col + warp * T, lane, T));
                 if (lane < nc) st_cluster(map_rank(smem_u32(mine + blockIdx.x), lane), v);
             }
-            cluster_barrier();
+            cluster_arrive();
+            if (warp >= NV) side(warp - NV);
+            cluster_wait();
             if (warp < NV) {
                 double v = lane < nc ? mine[lane] : 0.0;
 #pragma unroll
@@ -179,6 +190,8 @@ struct Group {
                     if (!ok) *bad = 1;
                 }
             }
+            else
+                side(warp - NV);
             __syncthreads();
             return *bad == 0;
         }
@@ -605,15 +618,18 @@ ResidentPlan plan_resident(int64_t rows, int width, size_t real, int sms, size_t
     return P;
 }
 
-template <typename R, int WW, bool MATS, bool CL, bool RECOMP>
-cudaError_t launch_resident(const ResidentPlan& P, const ResidentArgs<R>& a, int dev, cudaStream_t s)
+// Launches a resident kernel: as one cluster (CL) or cooperatively, so that
+// every CTA is resident.  cudaErrorCooperativeLaunchTooLarge when the device
+// (or a partition of it) has no room; nothing ran then.
+template <bool CL, typename Args>
+cudaError_t launch_group(void (*kernel)(Args), int ctas, int threads, size_t smem, const Args& a, int dev,
+                         cudaStream_t s)
 {
-    auto kernel = k_bicgstab_resident<R, WW, MATS, CL, RECOMP>;
     {
         static std::mutex mu;
-        static std::set<int> done;  // devices on which the kernel's attributes are set
+        static std::set<std::pair<int, const void*>> done;  // (device, kernel) whose attributes are set
         std::lock_guard<std::mutex> lock(mu);
-        if (!done.count(dev)) {
+        if (!done.count({dev, (const void*)kernel})) {
             int most = 0;
             cudaError_t e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
             cudaFuncAttributes fa{};
@@ -624,18 +640,18 @@ cudaError_t launch_resident(const ResidentPlan& P, const ResidentArgs<R>& a, int
             if (CL && e == cudaSuccess)
                 e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             if (e != cudaSuccess) return e;
-            done.insert(dev);
+            done.insert({dev, (const void*)kernel});
         }
     }
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(P.ctas);
-    cfg.blockDim = dim3(P.threads);
-    cfg.dynamicSmemBytes = P.smem;
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     if (CL) {
         at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = P.ctas;
+        at[0].val.clusterDim.x = ctas;
         at[0].val.clusterDim.y = 1;
         at[0].val.clusterDim.z = 1;
     }
@@ -646,9 +662,13 @@ cudaError_t launch_resident(const ResidentPlan& P, const ResidentArgs<R>& a, int
     cfg.attrs = at;
     cfg.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a);
-    // a device (or partition of one) without room for the cluster refuses it
-    // as the cooperative launch does
     return e == cudaErrorInvalidClusterSize ? cudaErrorCooperativeLaunchTooLarge : e;
+}
+
+template <typename R, int WW, bool MATS, bool CL, bool RECOMP>
+cudaError_t launch_resident(const ResidentPlan& P, const ResidentArgs<R>& a, int dev, cudaStream_t s)
+{
+    return launch_group<CL>(k_bicgstab_resident<R, WW, MATS, CL, RECOMP>, P.ctas, P.threads, P.smem, a, dev, s);
 }
 
 template <typename R, int WW>
