@@ -160,3 +160,25 @@ def test_resident_solve_iteration_cap():
     assert s.step(0.0, p.dt)["residual"] < 1e-12
     assert np.isfinite(s.state()[0]).all()
     s.close()
+
+
+@pytest.mark.parametrize("form,solver", [(L.FORM_FP64, "bicgstab"), (L.FORM_FP64, "gmres"), (L.FORM_MIXED, "bicgstab")])
+@pytest.mark.parametrize("N", [8, 64])
+def test_failed_assembly_leaves_the_state(form, solver, N):
+    """A non-positive diagonal is found by the solve's first kernel: the error
+    is reported, the traces stay as they were, and the next step works."""
+    p = _problem("heat2d", N)
+    p.config.form = form
+    s = problems.make_solver(p)
+    s.setup(tol=1e-13, max_iter=20000, linear_solver=solver)
+    before = s.state()[0]
+    s.set_coeff("D", -1e-3)
+    with pytest.raises(Exception, match="not positive"):
+        s.step(0.0, p.dt)
+    assert np.array_equal(s.state()[0], before)
+    s.set_coeff("D", 1.0)
+    m = OracleModel.from_problem(p)
+    s.step(0.0, p.dt)
+    m.step(0.0, p.dt, 1e-13)
+    assert rel_err(s.state()[0], m.Z_iF) < TOL_STATE
+    s.close()

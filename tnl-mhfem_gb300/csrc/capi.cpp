@@ -626,9 +626,12 @@ mhfem_status build_graph(mhfem_t h, bool fp32, int iters)
     return MHFEM_OK;
 }
 
+mhfem_status assembly_failed(mhfem_t h);
+
 mhfem_status status_from_krylov(mhfem_t h, const KrylovScalars& s, const char* what)
 {
     switch (s.status) {
+        case KS_ASSEMBLY: return assembly_failed(h);
         case KS_CONVERGED: return MHFEM_OK;
         case KS_MAXITER:
             return fail(h, MHFEM_ERR_NOT_CONVERGED,
@@ -645,9 +648,23 @@ double elapsed_s(std::chrono::steady_clock::time_point t0)
     return std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
 }
 
+mhfem_status assembly_failed(mhfem_t h)
+{
+    cudaMemsetAsync(h->err_flags, 0, sizeof(int32_t), h->stream);
+    return fail(h, MHFEM_ERR_NONPOSITIVE_DIAGONAL, "the diagonal matrix element is not positive");
+}
+
+// A resident launch wrote no result: a wait between its CTAs gave up.
+mhfem_status wait_gave_up(mhfem_t h, const char* what)
+{
+    CK(cudaMemsetAsync(h->W.counters, 0, kCounterWords * sizeof(uint32_t), h->stream));
+    return fail(h, MHFEM_ERR_CUDA, "%s: a grid barrier wait gave up", what);
+}
+
 mhfem_status status_from_gmres(mhfem_t h, const GmresCtl& c)
 {
     switch (c.status) {
+        case KS_ASSEMBLY: return assembly_failed(h);
         case KS_CONVERGED: return MHFEM_OK;
         case KS_MAXITER:
             return fail(h, MHFEM_ERR_NOT_CONVERGED,
@@ -661,7 +678,7 @@ mhfem_status status_from_gmres(mhfem_t h, const GmresCtl& c)
 // Restarted GMRES from the current Z_iF: CUDA graphs of check_every Arnoldi
 // iterations between host checks; at the end of each cycle the host runs the
 // small solve, the update of x and the restart from the true residual.
-mhfem_status run_gmres(mhfem_t h, double tol, int max_iter, int* iters, double* res)
+mhfem_status run_gmres(mhfem_t h, double tol, int max_iter, const int32_t* stop, int* iters, double* res)
 {
     const auto t0 = std::chrono::steady_clock::now();
     const int m = h->opts.gmres_restart;
@@ -684,56 +701,45 @@ mhfem_status run_gmres(mhfem_t h, double tol, int max_iter, int* iters, double* 
                            h->opts.gmres_restart_step_max};
     const bool adaptive = restart_adaptive(rule);
     int m_cur = m;
-    GmresState init{};
-    init.tol = tol;
-    init.m = m;
-    init.max_iter = max_iter;
-    init.m_min = rule.m_min;
-    init.m_max = rule.m_max;
-    init.step_min = rule.step_min;
-    init.step_max = rule.step_max;
-    init.max_cr = restart_max_cr();
-    init.min_cr = restart_min_cr();
-    CK(cudaMemcpyAsync(G.st, &init, sizeof(init), cudaMemcpyHostToDevice, h->stream));
-    gmres_init(h->A, h->rhs, h->Z_iF, G, h->W, true, h->stream);
+    const GmresStart start{tol, restart_max_cr(), restart_min_cr(), m, max_iter, rule.m_min, rule.m_max,
+                           rule.step_min, rule.step_max, stop};
+    gmres_init(h->A, h->rhs, h->Z_iF, G, h->W, &start, h->stream);
     h->launches += 1;
-    CK(cudaMemcpyAsync(G.host, &G.st->ctl, sizeof(GmresCtl), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
     CK(cudaGetLastError());
-    double res_prev = G.host->res;
     const bool reorth = h->opts.gmres_variant == MHFEM_GMRES_CGSR;
-    if (rows <= krylov_small_rows() && !G.host->done) {
+    if (rows <= krylov_small_rows()) {
         // the system fits: chunks of iterations, restarts included, in one
         // launch each (k_gmres_resident.cu), one host round trip per chunk;
         // the device applies the restart rule
-        CK(cudaMemcpyAsync(&G.st->res_prev, &res_prev, sizeof(double), cudaMemcpyHostToDevice, h->stream));
         constexpr int kChunk = 256;
-        bool small = true;
+        bool resident = true;
         for (bool first = true;; first = false) {
+            G.host->status = KS_PENDING;
             const cudaError_t e = gmres_resident(h->A, h->rhs, h->Z_iF, G, h->W, reorth, kChunk, h->stream);
             if (first && e == cudaErrorCooperativeLaunchTooLarge) {
                 // the device cannot hold the grid at once: nothing ran, the
                 // graph of iterations below goes on from the same state
                 cudaGetLastError();
-                small = false;
+                resident = false;
                 break;
             }
             CK(e);
             h->launches += 1;
-            CK(cudaMemcpyAsync(G.host, &G.st->ctl, sizeof(GmresCtl), cudaMemcpyDeviceToHost, h->stream));
-            CK(cudaMemcpyAsync(h->host_err, h->W.counters + kBarrierError, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
             CK(cudaStreamSynchronize(h->stream));
-            if (*h->host_err) return fail(h, MHFEM_ERR_CUDA, "GMRES (resident): a grid barrier wait gave up");
+            if (G.host->status == KS_PENDING) return wait_gave_up(h, "GMRES (resident)");
             if (G.host->done) break;
             if (h->opts.timeout_s > 0 && elapsed_s(t0) > h->opts.timeout_s)
                 return fail(h, MHFEM_ERR_TIMEOUT, "Krylov solve exceeded %.1f s", h->opts.timeout_s);
         }
-        if (small) {
+        if (resident) {
             *iters = G.host->it;
             *res = G.host->res;
             return status_from_gmres(h, *G.host);
         }
     }
+    CK(cudaMemcpyAsync(G.host, &G.st->ctl, sizeof(GmresCtl), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    double res_prev = G.host->res;
     if (!h->ggm) {
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
@@ -748,7 +754,7 @@ mhfem_status run_gmres(mhfem_t h, double tol, int max_iter, int* iters, double* 
         const bool restarted = G.host->cycle_end != 0;
         if (restarted) {
             gmres_update(h->Z_iF, G, rows, h->stream);
-            gmres_init(h->A, h->rhs, h->Z_iF, G, h->W, false, h->stream);
+            gmres_init(h->A, h->rhs, h->Z_iF, G, h->W, nullptr, h->stream);
             h->launches += 3;
             CK(cudaMemcpyAsync(G.host, &G.st->ctl, sizeof(GmresCtl), cudaMemcpyDeviceToHost, h->stream));
         }
@@ -779,44 +785,44 @@ mhfem_status run_gmres(mhfem_t h, double tol, int max_iter, int* iters, double* 
 }  // namespace
 
 // Runs FP64 BiCGStab from the current Z_iF until the device flag says done.
-mhfem_status mhfem::run_fp64(mhfem_t h, double tol, int max_iter, int* iters, double* res)
+mhfem_status mhfem::run_fp64(mhfem_t h, double tol, int max_iter, int* iters, double* res, const int32_t* stop)
 {
-    if (h->opts.linear_solver == MHFEM_SOLVER_GMRES) return run_gmres(h, tol, max_iter, iters, res);
+    if (h->opts.linear_solver == MHFEM_SOLVER_GMRES) return run_gmres(h, tol, max_iter, stop, iters, res);
     const auto t0 = std::chrono::steady_clock::now();
-    krylov_init_fp64(h->A, h->rhs, h->Z_iF, h->W, tol, max_iter, h->stream);
-    bool resident = krylov_resident_fits(h->A.rows, h->A.width, false);
-    if (resident) {
+    if (krylov_resident_fits(h->A.rows, h->A.width, false)) {
         // the system fits the SMs: chunks of iterations in one launch each
-        // (k_resident.cu), one host round trip per chunk
+        // (resident.cuh), one host round trip per chunk
         constexpr int kChunk = 256;
-        h->launches += 1;
         for (bool first = true;; first = false) {
-            const cudaError_t e = krylov_resident_fp64(h->A, h->Z_iF, h->W, kChunk, h->stream);
+            h->W.host_sc->status = KS_PENDING;
+            const cudaError_t e = krylov_resident_fp64(h->A, first ? h->rhs : nullptr, tol, max_iter, stop, h->Z_iF, h->W,
+                                                       h->W.host_sc, kChunk, h->stream);
             if (first && e == cudaErrorCooperativeLaunchTooLarge) {
                 // the device cannot hold the grid at once (a partitioned or
-                // shared GPU): nothing ran, so the five-kernel iteration
-                // below starts from the same initial state
+                // shared GPU): nothing ran, and the five-kernel iteration
+                // below takes the solve
                 cudaGetLastError();
-                resident = false;
                 break;
             }
             CK(e);
             h->launches += 1;
-            CK(cudaMemcpyAsync(h->W.host_sc, h->W.sc, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, h->stream));
-            CK(cudaMemcpyAsync(h->host_err, h->W.counters + kBarrierError, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
             CK(cudaStreamSynchronize(h->stream));
-            if (*h->host_err)
-                return fail(h, MHFEM_ERR_CUDA, "FP64 BiCGStab (resident): a grid barrier wait gave up");
-            if (h->W.host_sc->done) break;
+            if (h->W.host_sc->status == KS_PENDING) return wait_gave_up(h, "FP64 BiCGStab (resident)");
+            if (h->W.host_sc->done) {
+                *iters = h->W.host_sc->it;
+                *res = h->W.host_sc->res;
+                return status_from_krylov(h, *h->W.host_sc, "FP64 BiCGStab");
+            }
             if (h->opts.timeout_s > 0 && elapsed_s(t0) > h->opts.timeout_s)
                 return fail(h, MHFEM_ERR_TIMEOUT, "Krylov solve exceeded %.1f s", h->opts.timeout_s);
         }
-        if (resident) {
-            *iters = h->W.host_sc->it;
-            *res = h->W.host_sc->res;
-            return status_from_krylov(h, *h->W.host_sc, "FP64 BiCGStab");
-        }
     }
+    if (stop) {
+        CK(cudaMemcpyAsync(h->host_err, stop, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaStreamSynchronize(h->stream));
+        if (*h->host_err) return assembly_failed(h);
+    }
+    krylov_init_fp64(h->A, h->rhs, h->Z_iF, h->W, tol, max_iter, h->stream);
     CK(cudaMemcpyAsync(h->W.host_sc, h->W.sc, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     CK(cudaGetLastError());
@@ -839,22 +845,30 @@ mhfem_status mhfem::run_fp64(mhfem_t h, double tol, int max_iter, int* iters, do
 
 // FP32 inner BiCGStab on the FP32 copy of the matrix, FP64 outer residuals
 // and corrections, until the FP64 residual meets the tolerance.
-mhfem_status mhfem::run_mixed(mhfem_t h, int* iters, int* sweeps, double* res)
+mhfem_status mhfem::run_mixed(mhfem_t h, int* iters, int* sweeps, double* res, const int32_t* stop)
 {
     const auto t0 = std::chrono::steady_clock::now();
-    KrylovScalars init{};
-    init.tol = h->opts.tol;
-    init.max_iter = h->opts.max_sweeps;
-    CK(cudaMemcpyAsync(h->W.sc, &init, sizeof(init), cudaMemcpyHostToDevice, h->stream));
-    // the system fits the SMs: the inner iterations run resident (k_resident.cu)
+    // the system fits the SMs: the inner iterations run resident
+    // (resident.cuh), the first launch of a sweep queued behind its set-up, so
+    // that a sweep takes one host round trip
     bool resident = krylov_resident_fits(h->A.rows, h->A.width, true);
+    auto inner_resident = [&]() {
+        const cudaError_t e = krylov_resident_fp32(h->A, h->W, h->W.host_sc + 1, 256, h->stream);
+        if (e == cudaErrorCooperativeLaunchTooLarge) {
+            // the device cannot hold the launch at once: nothing ran
+            cudaGetLastError();
+            resident = false;
+            return cudaSuccess;
+        }
+        if (e == cudaSuccess) h->launches += 1;
+        return e;
+    };
     int total_inner = 0;
-    for (;;) {
-        mixed_outer_residual(h->A, h->rhs, h->Z_iF, h->W, h->opts.tol, h->opts.max_sweeps, h->stream);
+    for (bool begin = true;; begin = false) {
+        mixed_outer_residual(h->A, h->rhs, h->Z_iF, h->W, begin, h->opts.tol, h->opts.max_sweeps, stop, h->stream);
+        mixed_inner_init(h->W, h->opts.inner_tol, h->opts.inner_adaptive, h->opts.max_iter, resident, h->stream);
         h->launches += 2;
-        CK(cudaMemcpyAsync(h->W.host_sc, h->W.sc, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, h->stream));
-        mixed_inner_init(h->W, h->opts.inner_tol, h->opts.inner_adaptive, h->opts.max_iter, h->stream);
-        CK(cudaMemcpyAsync(h->W.host_sc + 1, h->W.sc32, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, h->stream));
+        if (resident) CK(inner_resident());
         CK(cudaStreamSynchronize(h->stream));
         CK(cudaGetLastError());
         const KrylovScalars outer = h->W.host_sc[0];
@@ -864,36 +878,26 @@ mhfem_status mhfem::run_mixed(mhfem_t h, int* iters, int* sweeps, double* res)
             *res = outer.res;
             return status_from_krylov(h, outer, "mixed-precision refinement");
         }
-        while (!h->W.host_sc[1].done) {
+        for (bool ran = resident; !h->W.host_sc[1].done; ran = true) {
+            if (resident && h->W.host_sc[1].status == KS_PENDING)
+                return wait_gave_up(h, "FP32 BiCGStab (resident)");
+            if (ran && h->opts.timeout_s > 0 && elapsed_s(t0) > h->opts.timeout_s)
+                return fail(h, MHFEM_ERR_TIMEOUT, "mixed solve exceeded %.1f s", h->opts.timeout_s);
             if (resident) {
-                const cudaError_t e = krylov_resident_fp32(h->A, h->W, 256, h->stream);
-                if (e == cudaErrorCooperativeLaunchTooLarge) {
-                    // the device cannot hold the launch at once: nothing ran
-                    cudaGetLastError();
-                    resident = false;
-                    continue;
-                }
-                CK(e);
-                h->launches += 1;
-                CK(cudaMemcpyAsync(h->W.host_sc + 1, h->W.sc32, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, h->stream));
-                CK(cudaMemcpyAsync(h->host_err, h->W.counters + kBarrierError, sizeof(int32_t), cudaMemcpyDeviceToHost,
-                                   h->stream));
-                CK(cudaStreamSynchronize(h->stream));
-                if (*h->host_err)
-                    return fail(h, MHFEM_ERR_CUDA, "FP32 BiCGStab (resident): a grid barrier wait gave up");
+                h->W.host_sc[1].status = KS_PENDING;
+                CK(inner_resident());
             }
-            else {
+            if (!resident) {
                 if (!h->g32) {
                     mhfem_status st = build_graph(h, true, h->opts.check_every);
                     if (st) return st;
                 }
                 CK(cudaGraphLaunch(h->g32, h->stream));
                 h->launches += 5 * h->g32_iters;
-                CK(cudaStreamSynchronize(h->stream));
             }
-            if (h->opts.timeout_s > 0 && elapsed_s(t0) > h->opts.timeout_s)
-                return fail(h, MHFEM_ERR_TIMEOUT, "mixed solve exceeded %.1f s", h->opts.timeout_s);
+            CK(cudaStreamSynchronize(h->stream));
         }
+        if (resident && h->W.host_sc[1].status == KS_PENDING) return wait_gave_up(h, "FP32 BiCGStab (resident)");
         const KrylovScalars inner = h->W.host_sc[1];
         total_inner += inner.it;
         if (inner.status == KS_NOTFINITE)
@@ -926,7 +930,7 @@ mhfem_status mhfem_pre_iterate(mhfem_t h, double t, double tau)
     h->cur_tau = tau;
     if ((st = run_hook(h, MHFEM_HOOK_PRE_ITERATE, t, tau)) != MHFEM_OK) return st;
     DevProblem P = make_problem(h);
-    cudaEventRecord(h->ev[0], h->stream);
+    if (h->timed) cudaEventRecord(h->ev[0], h->stream);
     if (h->hooks[MHFEM_HOOK_VECTOR_COEFFICIENTS].fn) {
         // Solver.hpp:627-652: this step's b first, then the model's
         // updateVectorCoefficients (its RT0 projections of u, w, a read b),
@@ -939,7 +943,7 @@ mhfem_status mhfem_pre_iterate(mhfem_t h, double t, double tau)
     }
     h->launches += launch_upwind(P, h->stream);
     h->launches += launch_cell_local(P, tau, h->stream);
-    cudaEventRecord(h->ev[1], h->stream);
+    if (h->timed) cudaEventRecord(h->ev[1], h->stream);
     CK(cudaGetLastError());
     return MHFEM_OK;
 }
@@ -953,7 +957,7 @@ mhfem_status mhfem_assemble(mhfem_t h, double t, double tau)
     cudaSetDevice(h->desc.device);
     DevProblem P = make_problem(h);
     h->launches += launch_assemble(P, h->amap, h->A, h->rhs, h->fp32_copy, h->stream);
-    cudaEventRecord(h->ev[2], h->stream);
+    if (h->timed) cudaEventRecord(h->ev[2], h->stream);
     CK(cudaGetLastError());
     return MHFEM_OK;
 }
@@ -964,12 +968,13 @@ mhfem_status mhfem_solve(mhfem_t h, mhfem_step_stats* stats)
     if (st) return st;
     if (!h->pattern_ready) return fail(h, MHFEM_ERR_STATE, "the linear system is not assembled");
     cudaSetDevice(h->desc.device);
-    // assembly error word (non-positive or non-finite diagonal)
-    CK(cudaMemcpyAsync(h->host_err, h->err_flags, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    if (*h->host_err) {
-        cudaMemsetAsync(h->err_flags, 0, sizeof(int32_t), h->stream);
-        return fail(h, MHFEM_ERR_NONPOSITIVE_DIAGONAL, "the diagonal matrix element is not positive");
+    // the assembly's error word (non-positive or non-finite diagonal): the
+    // solve's first kernel reads it and leaves everything as it is; the
+    // learned form works on the system before its solve, so there the host asks
+    if (h->desc.form == MHFEM_FORM_LEARNED) {
+        CK(cudaMemcpyAsync(h->host_err, h->err_flags, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaStreamSynchronize(h->stream));
+        if (*h->host_err) return assembly_failed(h);
     }
     int iters = 0, sweeps = 1;
     double res = 0;
@@ -982,10 +987,10 @@ mhfem_status mhfem_solve(mhfem_t h, mhfem_step_stats* stats)
         stats->base_residual = -1;
         stats->guess_source = 0;
     }
-    if (h->desc.form == MHFEM_FORM_MIXED) st = run_mixed(h, &iters, &sweeps, &res);
+    if (h->desc.form == MHFEM_FORM_MIXED) st = run_mixed(h, &iters, &sweeps, &res, h->err_flags);
     else if (h->desc.form == MHFEM_FORM_LEARNED) st = learned_solve(h, &iters, &sweeps, &res, stats);
-    else st = run_fp64(h, h->opts.tol, h->opts.max_iter, &iters, &res);
-    cudaEventRecord(h->ev[3], h->stream);
+    else st = run_fp64(h, h->opts.tol, h->opts.max_iter, &iters, &res, h->err_flags);
+    if (h->timed) cudaEventRecord(h->ev[3], h->stream);
     h->total_iters += iters;
     if (stats) {
         stats->iterations = iters;
@@ -1002,7 +1007,7 @@ mhfem_status mhfem_post_iterate(mhfem_t h, double t, double tau)
     cudaSetDevice(h->desc.device);
     DevProblem P = make_problem(h);
     h->launches += launch_reconstruct(P, h->stream);
-    cudaEventRecord(h->ev[4], h->stream);
+    if (h->timed) cudaEventRecord(h->ev[4], h->stream);
     CK(cudaGetLastError());
     return run_hook(h, MHFEM_HOOK_POST_ITERATE, t, tau);
 }
@@ -1042,11 +1047,14 @@ mhfem_status mhfem_array_device(mhfem_t h, int32_t which, double** data, int64_t
 
 mhfem_status mhfem_step(mhfem_t h, double t, double tau, mhfem_step_stats* stats)
 {
-    mhfem_status st;
-    if ((st = mhfem_pre_iterate(h, t, tau)) != MHFEM_OK) return st;
-    if ((st = mhfem_assemble(h, t, tau)) != MHFEM_OK) return st;
-    if ((st = mhfem_solve(h, stats)) != MHFEM_OK) return st;
-    if ((st = mhfem_post_iterate(h, t, tau)) != MHFEM_OK) return st;
+    if (!h) return MHFEM_ERR_INVALID_ARGUMENT;
+    h->timed = stats != nullptr;  // the events between the phases are for the step's statistics
+    mhfem_status st = mhfem_pre_iterate(h, t, tau);
+    if (st == MHFEM_OK) st = mhfem_assemble(h, t, tau);
+    if (st == MHFEM_OK) st = mhfem_solve(h, stats);
+    if (st == MHFEM_OK) st = mhfem_post_iterate(h, t, tau);
+    h->timed = false;
+    if (st != MHFEM_OK) return st;
     h->total_steps += 1;
     if (stats) {
         CK(cudaEventSynchronize(h->ev[4]));

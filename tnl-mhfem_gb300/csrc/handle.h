@@ -80,6 +80,7 @@ struct mhfem_solver_s {
         void* user = nullptr;
     } hooks[3];              // MHFEM_HOOK_PRE_ITERATE, MHFEM_HOOK_POST_ITERATE, MHFEM_HOOK_VECTOR_COEFFICIENTS
     bool guess_timed = false;
+    bool timed = false;      // record the phase events (a step that returns statistics)
     std::vector<void*> allocs;
 
     // host copies: the coordinates and (learned form) D, f, psi build the
@@ -133,10 +134,12 @@ inline void dfree(mhfem_t h, T*& p)
     p = nullptr;
 }
 
-// FP64 BiCGStab from the current Z_iF (capi.cpp).
-mhfem_status run_fp64(mhfem_t h, double tol, int max_iter, int* iters, double* res);
+// FP64 BiCGStab or GMRES from the current Z_iF (capi.cpp).  A non-zero word at
+// `stop` (device memory, may be null) ends the solve before it changes
+// anything, with the assembly's error.
+mhfem_status run_fp64(mhfem_t h, double tol, int max_iter, int* iters, double* res, const int32_t* stop = nullptr);
 // Mixed-precision refinement from the current Z_iF (capi.cpp); needs fp32_copy.
-mhfem_status run_mixed(mhfem_t h, int* iters, int* sweeps, double* res);
+mhfem_status run_mixed(mhfem_t h, int* iters, int* sweeps, double* res, const int32_t* stop = nullptr);
 // Learned form (learned.cpp): the gate, the solve (FP64 or mixed) and online training.
 mhfem_status learned_solve(mhfem_t h, int* iters, int* sweeps, double* res, mhfem_step_stats* stats);
 void learned_release(mhfem_t h);

@@ -51,8 +51,17 @@ static_assert(kGmDots <= kGmStride && kGmDots <= KB, "GMRES dot products per blo
 template <int WW>
 __global__ void __launch_bounds__(KB) k_gm_init(const int32_t* cols, const double* vals, int W, int64_t rows,
                                                 const double* b, const double* x, double* U, GmresState* st,
-                                                int first, double* partials, uint32_t* counter)
+                                                int first, const GmresStart start, double* partials,
+                                                uint32_t* counter)
 {
+    if (first && start.stop && *start.stop) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            st->ctl = GmresCtl{};
+            st->ctl.status = KS_ASSEMBLY;
+            st->ctl.done = 1;
+        }
+        return;
+    }
     double acc[2] = {0, 0};
     for (int64_t q = (int64_t)blockIdx.x * KB + threadIdx.x; q < rows; q += (int64_t)gridDim.x * KB) {
         const double bq = b[q];
@@ -74,12 +83,22 @@ __global__ void __launch_bounds__(KB) k_gm_init(const int32_t* cols, const doubl
             c.it = 0;
             c.status = KS_RUNNING;
             c.done = 0;
+            st->tol = start.tol;
+            st->m = start.m;
+            st->max_iter = start.max_iter;
+            st->m_min = start.m_min;
+            st->m_max = start.m_max;
+            st->step_min = start.step_min;
+            st->step_max = start.step_max;
+            st->max_cr = start.max_cr;
+            st->min_cr = start.min_cr;
         }
         const double beta = sqrt(s[0]);
         c.res = beta / c.bnorm;
         st->g[0] = beta;
         st->inv[0] = beta > 0 ? 1.0 / beta : 0.0;
         st->j = 0;
+        st->res_prev = c.res;
         c.cycle_end = 0;
         if (!finite(c.res)) { c.status = KS_NOTFINITE; c.done = 1; }
         else if (c.res < st->tol) { c.status = KS_CONVERGED; c.done = 1; }
@@ -280,12 +299,12 @@ __global__ void __launch_bounds__(KB) k_gm_update_x(int64_t rows, const double* 
 
 // ---- launchers --------------------------------------------------------------
 
-void gmres_init(const EllMatrix& A, const double* b, const double* x, GmresWork& G, KrylovWork& W, bool first,
-                cudaStream_t s)
+void gmres_init(const EllMatrix& A, const double* b, const double* x, GmresWork& G, KrylovWork& W,
+                const GmresStart* start, cudaStream_t s)
 {
     MHFEM_WIDTH_DISPATCH(A.width, (k_gm_init<WW><<<row_grid(k_gm_init<WW>, A.rows), KB, 0, s>>>(
-                                      A.cols, A.vals, A.width, A.rows, b, x, G.U, G.st, first ? 1 : 0, W.partials,
-                                      W.counters)));
+                                      A.cols, A.vals, A.width, A.rows, b, x, G.U, G.st, start ? 1 : 0,
+                                      start ? *start : GmresStart{}, W.partials, W.counters)));
 }
 
 void gmres_iterate(const EllMatrix& A, GmresWork& G, KrylovWork& W, int iters, bool reorth, cudaStream_t s)

@@ -51,6 +51,7 @@ struct GmresArgs {
     const double* b;
     double *x, *U;
     GmresState* st;
+    GmresCtl* host;     // pinned copy of st->ctl
     double* pdots;      // [2][CTA][kDots]
     double* partials;
     unsigned int* bar;
@@ -105,7 +106,10 @@ __global__ void __launch_bounds__(kGmresThreads, 1) k_gmres_resident(const Gmres
         if (threadIdx.x == 0) bad = 0;
     }
     __syncthreads();
-    if (S.ctl.done) return;  // the same in every CTA
+    if (S.ctl.done) {  // the same in every CTA
+        if (blockIdx.x == 0 && threadIdx.x == 0) *g.host = S.ctl;
+        return;
+    }
     if (threadIdx.x == 0) inv_bnorm = 1.0 / S.ctl.bnorm;
 
     double* col = smem;
@@ -125,6 +129,7 @@ __global__ void __launch_bounds__(kGmresThreads, 1) k_gmres_resident(const Gmres
             }
     }
     Group<CL> G{col, tot, slots, &bad, g.partials, g.bar, g.bar_err};
+    G.begin();
     if constexpr (CL) cluster_barrier();
     else __syncthreads();
 
@@ -394,7 +399,9 @@ __global__ void __launch_bounds__(kGmresThreads, 1) k_gmres_resident(const Gmres
             for (int i = 0; i <= S.j; ++i)
                 for (int m = threadIdx.x; m < n; m += T) g.U[(int64_t)i * rows + base + m] = su[i * rc + m];
     }
+    G.end();
     if (blockIdx.x == 0) {
+        if (threadIdx.x == 0) *g.host = S.ctl;
         const unsigned long long* src = reinterpret_cast<const unsigned long long*>(&S);
         unsigned long long* dst = reinterpret_cast<unsigned long long*>(g.st);
         for (int k = threadIdx.x; k < (int)(sizeof(GmresState) / 8); k += T) dst[k] = src[k];
@@ -463,9 +470,7 @@ cudaError_t gmres_resident(const EllMatrix& A, const double* b, double* x, Gmres
     if ((int64_t)3 * kSums * P.ctas > (int64_t)W.grid * kPartStride ||
         (int64_t)2 * P.ctas * kDots > (int64_t)krylov_grid() * kGmStride)
         return cudaErrorCooperativeLaunchTooLarge;
-    e = cudaMemsetAsync(W.counters, 0, kCounterWords * sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
-    const GmresArgs a{A.cols, A.vals, A.width, A.rows, P.rc, reorth ? 1 : 0, G.m + 1, b, x, G.U, G.st, G.partials,
+    const GmresArgs a{A.cols, A.vals, A.width, A.rows, P.rc, reorth ? 1 : 0, G.m + 1, b, x, G.U, G.st, G.host, G.partials,
                       W.partials, W.counters + kBarrierFirst, reinterpret_cast<int*>(W.counters + kBarrierError), iters};
     MHFEM_WIDTH_DISPATCH(A.width, e = launch_gmres_form<WW>(P, a, dev, s));
     return e;

@@ -1044,9 +1044,17 @@ void residual_norm_fp64(const EllMatrix& A, const double* b, const double* x, Kr
 template <int WW>
 __global__ void __launch_bounds__(KB) k_outer_residual(const int32_t* cols, const double* vals, int W,
                                                        int64_t rows, const double* b, const double* x,
-                                                       double* r, KrylovScalars* sc, double* partials,
+                                                       double* r, KrylovScalars* sc, int begin, double tol,
+                                                       int max_sweeps, const int32_t* stop, double* partials,
                                                        uint32_t* counter)
 {
+    if (begin && stop && *stop) {  // the assembly failed: nothing is solved
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            sc->status = KS_ASSEMBLY;
+            sc->done = 1;
+        }
+        return;
+    }
     double acc[2] = {0, 0};
     for (int64_t q = (int64_t)blockIdx.x * KB + threadIdx.x; q < rows; q += (int64_t)gridDim.x * KB) {
         const double rv = b[q] - spmv_row<double, WW>(cols, vals, W, rows, q, x);
@@ -1064,6 +1072,12 @@ __global__ void __launch_bounds__(KB) k_outer_residual(const int32_t* cols, cons
         sc->bnorm = bn;
         sc->snorm = sqrt(s[0]);
         sc->res = sc->snorm / bn;
+        if (begin) {
+            sc->tol = tol;
+            sc->max_iter = max_sweeps;
+            sc->it = 0;
+            sc->status = KS_RUNNING;
+        }
         sc->it += 1;  // refinement sweep counter
         sc->done = 0;
         if (!finite(sc->res)) { sc->status = KS_NOTFINITE; sc->done = 1; }
@@ -1076,7 +1090,8 @@ __global__ void __launch_bounds__(KB) k_outer_residual(const int32_t* cols, cons
 __global__ void __launch_bounds__(KB) k_inner_init(int64_t rows, const double* r, float* r32, float* rh32,
                                                    float* p32, float* x32, const KrylovScalars* outer,
                                                    KrylovScalars* sc, double inner_tol, int adaptive, int max_iter,
-                                                   double* partials, uint32_t* counter)
+                                                   KrylovScalars* host, int pending, double* partials,
+                                                   uint32_t* counter)
 {
     const double scale = (outer->snorm > 0) ? 1.0 / outer->snorm : 0.0;
     float acc[1] = {0.f};
@@ -1108,6 +1123,9 @@ __global__ void __launch_bounds__(KB) k_inner_init(int64_t rows, const double* r
         sc->snorm = 1.0;
         sc->status = KS_RUNNING;
         sc->done = (outer->done || s[0] == 0) ? 1 : 0;
+        host[0] = *outer;
+        host[1] = *sc;
+        if (pending) host[1].status = KS_PENDING;
     }
 }
 
@@ -1120,18 +1138,17 @@ __global__ void __launch_bounds__(KB) k_apply_correction(int64_t rows, double* x
         x[q] = fma(scale, f32_to_f64(x32[q]), x[q]);
 }
 
-void mixed_outer_residual(const EllMatrix& A, const double* b, const double* x, KrylovWork& W,
-                          double tol, int max_sweeps, cudaStream_t s)
+void mixed_outer_residual(const EllMatrix& A, const double* b, const double* x, KrylovWork& W, bool begin,
+                          double tol, int max_sweeps, const int32_t* stop, cudaStream_t s)
 {
-    (void)tol; (void)max_sweeps;
     MHFEM_WIDTH_DISPATCH(A.width, (k_outer_residual<WW><<<row_grid(k_outer_residual<WW>, A.rows), KB, 0, s>>>(A.cols, A.vals, A.width, A.rows, b,
-                                                 x, W.r, W.sc, W.partials, W.counters)));
+                                                 x, W.r, W.sc, begin ? 1 : 0, tol, max_sweeps, stop, W.partials, W.counters)));
 }
 
-void mixed_inner_init(KrylovWork& W, double inner_tol, int adaptive, int max_iter, cudaStream_t s)
+void mixed_inner_init(KrylovWork& W, double inner_tol, int adaptive, int max_iter, bool pending, cudaStream_t s)
 {
     k_inner_init<<<row_grid(k_inner_init, W.rows), KB, 0, s>>>(W.rows, W.r, W.r32, W.rh32, W.p32, W.x32, W.sc, W.sc32, inner_tol,
-                                       adaptive, max_iter, W.partials, W.counters);
+                                       adaptive, max_iter, W.host_sc, pending ? 1 : 0, W.partials, W.counters);
 }
 
 void krylov_iterate_fp32(const EllMatrix& A, KrylovWork& W, int iters, cudaStream_t s)

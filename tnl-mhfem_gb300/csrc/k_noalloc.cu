@@ -132,38 +132,42 @@ extern "C" mhfem_status mhfem_bicgstab_noalloc(const int32_t* cols, const double
         if (cudaStreamSynchronize(s) != cudaSuccess) return MHFEM_ERR_CUDA;
         if (bad != 0) return MHFEM_ERR_INVALID_ARGUMENT;  // a column outside [0, rows): nothing else was queued
     }
-    mhfem::krylov_init_fp64(A, rhs, x, W, tol, max_iter, s);
-    if (cudaGetLastError() != cudaSuccess) return MHFEM_ERR_CUDA;
     bool resident = mhfem::krylov_resident_fits(rows, width, false);  // on a whole GPU always, at this size limit
     mhfem::KrylovScalars hs{};
     int32_t barrier_failed = 0;
     for (bool first = true;; first = false) {
-        if (cudaMemcpyAsync(&hs, W.sc, sizeof(hs), cudaMemcpyDeviceToHost, s) != cudaSuccess) return MHFEM_ERR_CUDA;
-        if (resident && cudaMemcpyAsync(&barrier_failed, W.counters + mhfem::kBarrierError, sizeof(barrier_failed), cudaMemcpyDeviceToHost,
-                                     s) != cudaSuccess)
-            return MHFEM_ERR_CUDA;
-        if (cudaStreamSynchronize(s) != cudaSuccess) return MHFEM_ERR_CUDA;
-        if (barrier_failed) return MHFEM_ERR_CUDA;  // a grid barrier wait ran out (the context stays usable)
-        if (hs.done) break;
-        // the stream has drained here, so the shared scratch is idle when the limit ends the call
-        if (timeout_s > 0 && elapsed_s(t0) > timeout_s) {
+        if (!first && timeout_s > 0 && elapsed_s(t0) > timeout_s) {
+            // the stream has drained, so the shared scratch is idle when the limit ends the call
             if (iterations) *iterations = hs.it;
             if (residual) *residual = hs.res;
             return MHFEM_ERR_TIMEOUT;
         }
         if (resident) {
-            const cudaError_t e = mhfem::krylov_resident_fp64(A, x, W, 256, s);
+            // a limit that has passed already: the first residual alone
+            const int chunk = timeout_s > 0 && elapsed_s(t0) > timeout_s ? 0 : 256;
+            const cudaError_t e = mhfem::krylov_resident_fp64(A, first ? rhs : nullptr, tol, max_iter, nullptr, x, W,
+                                                              nullptr, chunk, s);
             if (first && e == cudaErrorCooperativeLaunchTooLarge) {
                 // the device cannot hold the grid at once (a partitioned or
-                // shared GPU): nothing ran, the five-kernel iteration goes on
+                // shared GPU): nothing ran, the five-kernel iteration takes over
                 cudaGetLastError();
                 resident = false;
             }
             else if (e != cudaSuccess)
                 return MHFEM_ERR_CUDA;
         }
-        if (!resident) mhfem::krylov_iterate_fp64(A, x, W, 8, s);
+        if (!resident) {
+            if (first) mhfem::krylov_init_fp64(A, rhs, x, W, tol, max_iter, s);
+            else mhfem::krylov_iterate_fp64(A, x, W, 8, s);
+        }
         if (cudaGetLastError() != cudaSuccess) return MHFEM_ERR_CUDA;
+        if (cudaMemcpyAsync(&hs, W.sc, sizeof(hs), cudaMemcpyDeviceToHost, s) != cudaSuccess) return MHFEM_ERR_CUDA;
+        if (resident && cudaMemcpyAsync(&barrier_failed, W.counters + mhfem::kBarrierError, sizeof(barrier_failed),
+                                        cudaMemcpyDeviceToHost, s) != cudaSuccess)
+            return MHFEM_ERR_CUDA;
+        if (cudaStreamSynchronize(s) != cudaSuccess) return MHFEM_ERR_CUDA;
+        if (barrier_failed) return MHFEM_ERR_CUDA;  // a grid barrier wait ran out (the context stays usable)
+        if (hs.done) break;
     }
     if (iterations) *iterations = hs.it;
     if (residual) *residual = hs.res;

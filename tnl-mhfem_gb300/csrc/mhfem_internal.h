@@ -30,7 +30,10 @@ struct KrylovScalars {
 };
 
 // Krylov status codes written to KrylovScalars::status.
-enum : int32_t { KS_RUNNING = 0, KS_CONVERGED = 1, KS_MAXITER = 2, KS_BREAKDOWN = 3, KS_NOTFINITE = 4 };
+// KS_ASSEMBLY: the assembly reported a non-positive diagonal, nothing was
+// solved; KS_PENDING: a pinned copy that its launch has not written.
+enum : int32_t { KS_RUNNING = 0, KS_CONVERGED = 1, KS_MAXITER = 2, KS_BREAKDOWN = 3, KS_NOTFINITE = 4,
+                 KS_ASSEMBLY = 5, KS_PENDING = -1 };
 
 #ifdef __CUDACC__
 // 1 / d in FP64 for the row scaling of the assembly and the LU pivots of the
@@ -201,16 +204,25 @@ struct GmresWork {
     int32_t* host_m = nullptr;    // pinned: the next cycle's restart length (adaptive restarting)
 };
 
-// r = b - A x into u_0 and the restart scalars; first: also ||b|| and it = 0
+// What begins a GMRES solve: the tolerance, the restart lengths and their
+// rule (GmresState), the word that stops it (see krylov_resident_fp64).
+struct GmresStart {
+    double tol, max_cr, min_cr;
+    int32_t m, max_iter, m_min, m_max, step_min, step_max;
+    const int32_t* stop;
+};
+// r = b - A x into u_0 and the restart scalars; start not null: also ||b|| and
+// the whole state (it = 0)
 void gmres_init(const EllMatrix& A, const double* b, const double* x, GmresWork& G, KrylovWork& W,
-                bool first, cudaStream_t s);
+                const GmresStart* start, cudaStream_t s);
 // `iters` Arnoldi iterations (each returns at once after the cycle ended)
 void gmres_iterate(const EllMatrix& A, GmresWork& G, KrylovWork& W, int iters, bool reorth, cudaStream_t s);
 // end of a cycle: solve the triangular system and update x
 void gmres_update(double* x, GmresWork& G, int64_t rows, cudaStream_t s);
 // Small systems (at most krylov_small_rows() rows): up to `iters` Arnoldi
-// iterations, restarts included, in one launch (k_gmres_resident.cu; the flag
-// at W.counters + kBarrierError as for krylov_resident_fp64).
+// iterations, restarts included, in one launch (k_gmres_resident.cu) on a
+// solve set up by gmres_init; G.host gets the control words, as *host of
+// krylov_resident_fp64 the scalars.
 cudaError_t gmres_resident(const EllMatrix& A, const double* b, double* x, GmresWork& G, KrylovWork& W, bool reorth,
                            int iters, cudaStream_t s);
 void krylov_iterate_fp64(const EllMatrix& A, double* x, KrylovWork& W, int iters, cudaStream_t s);
@@ -218,30 +230,40 @@ void krylov_iterate_fp64(const EllMatrix& A, double* x, KrylovWork& W, int iters
 int64_t krylov_small_rows();
 // Words of KrylovWork::counters: [0] the reductions' ticket, [3] the flag of a
 // resident solve's wait that gave up, then the resident solves' four arrival
-// counters, each on a 128-byte line of its own.
+// counters, each on a 128-byte line of its own with the count at the end of
+// the last launch behind it.  Zero before the first launch and after one whose
+// wait gave up.
 constexpr int kBarrierError = 3;
 constexpr int kBarrierFirst = 32;
 constexpr int kBarrierStride = 32;
 constexpr int kCounterWords = kBarrierFirst + 4 * kBarrierStride;
 // Whether a system of this size can run resident on the SMs of the current
-// device (k_resident.cu), and up to `iters` FP64 BiCGStab iterations of it in
-// one launch on a solve set up by krylov_init_fp64 (W.r, W.rh, W.p; W.v and
-// W.s are written).  The flag at W.counters + kBarrierError is non-zero after
-// a wait between its CTAs gave up.  cudaErrorCooperativeLaunchTooLarge: the
-// device cannot hold the launch at once, and nothing ran.
+// device (resident.cuh).
 bool krylov_resident_fits(int64_t rows, int width, bool fp32);
-cudaError_t krylov_resident_fp64(const EllMatrix& A, double* x, KrylovWork& W, int iters, cudaStream_t s);
+// Up to `iters` FP64 BiCGStab iterations of A x = b in one launch, which also
+// forms the first residual (b not null: tol, max_iter and the solve's state
+// begin; *stop non-zero: it ends at once with KS_ASSEMBLY and x untouched), or
+// goes on with the solve (b null).  W.r, W.rh, W.p, W.v and W.s are work
+// vectors.  The scalars end in W.sc and, when `host` (pinned) is not null, in
+// *host; a launch one of whose waits gave up sets the flag at W.counters +
+// kBarrierError and writes neither.  cudaErrorCooperativeLaunchTooLarge: the
+// device cannot hold the launch at once, and nothing ran.
+cudaError_t krylov_resident_fp64(const EllMatrix& A, const double* b, double tol, int max_iter, const int32_t* stop,
+                                 double* x, KrylovWork& W, KrylovScalars* host, int iters, cudaStream_t s);
 // The same for the mixed form's inner solve, set up by mixed_inner_init.
-cudaError_t krylov_resident_fp32(const EllMatrix& A, KrylovWork& W, int iters, cudaStream_t s);
+cudaError_t krylov_resident_fp32(const EllMatrix& A, KrylovWork& W, KrylovScalars* host, int iters, cudaStream_t s);
 // One cooperative launch of `ctas` CTAs through the persistent solves'
 // bounded grid barrier, CTA `skip` (none if negative) never arriving; counts
 // the CTAs that passed and that gave up, and returns the failure flag.
 cudaError_t grid_barrier_check(int ctas, int skip, unsigned int max_polls, int* passed, int* gave_up, int* flag);
 
 // mixed: outer residual r = b - A x (FP64) -> sc; scale into r32; inner FP32 solve; x += scale*e
-void mixed_outer_residual(const EllMatrix& A, const double* b, const double* x, KrylovWork& W,
-                          double tol, int max_sweeps, cudaStream_t s);
-void mixed_inner_init(KrylovWork& W, double inner_tol, int adaptive, int max_iter, cudaStream_t s);
+// begin: the first sweep, which sets the outer scalars up (tol, max_sweeps; stop as for krylov_resident_fp64)
+void mixed_outer_residual(const EllMatrix& A, const double* b, const double* x, KrylovWork& W, bool begin,
+                          double tol, int max_sweeps, const int32_t* stop, cudaStream_t s);
+// W.host_sc[0] gets the outer scalars and W.host_sc[1] the inner ones, the
+// latter marked KS_PENDING when an inner launch that writes them follows
+void mixed_inner_init(KrylovWork& W, double inner_tol, int adaptive, int max_iter, bool pending, cudaStream_t s);
 void krylov_iterate_fp32(const EllMatrix& A, KrylovWork& W, int iters, cudaStream_t s);
 void mixed_apply_correction(double* x, KrylovWork& W, cudaStream_t s);
 

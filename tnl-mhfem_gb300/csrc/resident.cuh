@@ -56,7 +56,12 @@ struct ResidentArgs {
     int rc;             // rows per CTA
     int x_in_smem;
     T *x, *r, *rh, *p, *v, *s;
+    const T* b;             // right-hand side: the launch begins the solve (r = b - A x); null: it goes on
+    double tol;             // with b: the solve's limits
+    int max_iter;
+    const int32_t* stop;    // with b: non-zero word: end at once with KS_ASSEMBLY (may be null)
     KrylovScalars* sc;
+    KrylovScalars* host;    // pinned copy of sc for the host (may be null)
     double* partials;   // [3 reductions][kSums][CTA]
     unsigned int* bar;  // kSums arrival counters, kBarrierStride words apart
     int* bar_err;
@@ -126,7 +131,22 @@ struct Group {
     double* partials;
     unsigned int* bar;
     int* err;
-    unsigned int target = 0;  // arrivals this thread's counter (its warp's) has seen
+    // Arrivals that this thread's counter (its warp's) has seen.  The counts
+    // run on from launch to launch: the word behind a counter holds its value
+    // at the last launch's end.
+    unsigned int target = 0;
+
+    __device__ __forceinline__ void begin()
+    {
+        const int warp = threadIdx.x >> 5;
+        if (!CL && warp < kSums) target = __ldcg(bar + warp * kBarrierStride + 1);
+    }
+    // Call once every CTA has passed the launch's last wait.
+    __device__ __forceinline__ void end()
+    {
+        const int warp = threadIdx.x >> 5;
+        if (!CL && blockIdx.x == 0 && warp < kSums && (threadIdx.x & 31) == 0) bar[warp * kBarrierStride + 1] = target;
+    }
 
     // tot[q] = the sum of every thread's acc[q]; also a barrier that makes
     // the global (or cluster-shared) writes before it visible after it.
@@ -293,13 +313,31 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
     const int64_t base = (int64_t)blockIdx.x * rc, rows = g.rows;
     const int n = (int)max((int64_t)0, min((int64_t)rc, rows - base));
     __shared__ EndLimits limits;
+    const bool first = g.b != nullptr;
     if (threadIdx.x == 0) {
-        S = *g.sc;
-        limits = end_limits(S);
+        if (first) {
+            S = KrylovScalars{};
+            S.tol = g.tol;
+            S.max_iter = g.max_iter;
+            if (g.stop && *g.stop) {
+                S.status = KS_ASSEMBLY;
+                S.done = 1;
+            }
+        }
+        else {
+            S = *g.sc;
+            limits = end_limits(S);
+        }
         bad = 0;
     }
     __syncthreads();
-    if (S.done) return;  // the same in every CTA
+    if (S.done) {  // the same in every CTA
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            *g.sc = S;
+            if (g.host) *g.host = S;
+        }
+        return;
+    }
 
     double* col = smem;
     R* sr = reinterpret_cast<R*>(col + kSums * T);
@@ -317,9 +355,11 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
     uint32_t* scol = reinterpret_cast<uint32_t*>(sa + (int64_t)(MATS ? W : 0) * rc);
 
     for (int m = threadIdx.x; m < n; m += T) {
-        sr[m] = __ldcg(g.r + base + m);
-        srh[m] = __ldcg(g.rh + base + m);
-        sp[m] = __ldcg(g.p + base + m);
+        if (!first) {
+            sr[m] = __ldcg(g.r + base + m);
+            srh[m] = __ldcg(g.rh + base + m);
+            sp[m] = __ldcg(g.p + base + m);
+        }
         if (g.x_in_smem) xp[m] = g.x[base + m];
     }
     if constexpr (MATS)
@@ -332,6 +372,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
                 scol[k * rc + m] = CL ? map_rank(smem_u32(sr + c % rc), c / rc) : c;
             }
     Group<CL> G{col, tot, slots, &bad, g.partials, g.bar, g.bar_err};
+    G.begin();
     if constexpr (CL) cluster_barrier();  // every CTA's shared memory is set up
     else __syncthreads();
 
@@ -412,7 +453,41 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
     };
     const uint32_t off_p = (uint32_t)((char*)sp - (char*)sr), off_v = (uint32_t)((char*)sv - (char*)sr);
 
-    for (int k = 0; k < g.max_its; ++k) {
+    if (first) {
+        // rh = p = r = b - A x (x gathered from memory), ||r||, ||b||
+        R acc[2] = {0, 0};
+        for (int m = threadIdx.x; m < n; m += T) {
+            R y = g.x[base + m];
+            for (int k = 0; k < W; ++k) {
+                const int64_t o = (int64_t)k * rows + base + m;
+                y = fma(MATS ? sa[k * rc + m] : __ldg(g.vals + o), g.x[__ldg(g.cols + o)], y);
+            }
+            const R bm = g.b[base + m], rv = bm - y;
+            sr[m] = rv;
+            srh[m] = rv;
+            sp[m] = rv;
+            if (!CL) {
+                __stcg(g.p + base + m, rv);
+                if (RECOMP) __stcg(g.r + base + m, rv);
+            }
+            acc[0] = fma(rv, rv, acc[0]);
+            acc[1] = fma(bm, bm, acc[1]);
+        }
+        if (!G.reduce(acc, 2)) return;
+        if (threadIdx.x == 0) {
+            const double rn = sqrt(tot[0]), bn = sqrt(tot[1]);
+            S.bnorm = bn == 0 ? 1.0 : bn;
+            S.rho = S.rr = tot[0];
+            S.rhnorm = rn;
+            S.res = rn / S.bnorm;
+            if (!finite(S.res)) { S.status = KS_NOTFINITE; S.done = 1; }
+            else if (S.res < S.tol) { S.status = KS_CONVERGED; S.done = 1; }
+            limits = end_limits(S);
+        }
+        __syncthreads();
+    }
+
+    for (int k = 0; k < g.max_its && !S.done; ++k) {
         // A. v = A p, (rh, v) -> alpha
         {
             R acc[1] = {0};
@@ -551,7 +626,11 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
         g.rh[base + m] = srh[m];
         g.p[base + m] = sp[m];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *g.sc = S;
+    G.end();
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *g.sc = S;
+        if (g.host) *g.host = S;
+    }
     if constexpr (CL) cluster_barrier();  // no CTA leaves while another may still read its shared memory
 }
 
@@ -692,19 +771,20 @@ cudaError_t device_plan(int64_t rows, int width, size_t real, int* dev, Resident
     return cudaSuccess;
 }
 
+// b: begins the solve of A x = b (tol, max_iter, stop); null: goes on with it.
 template <typename R>
-cudaError_t iterate_resident(const EllMatrix& A, const R* vals, R* x, R* r, R* rh, R* p, R* v, R* sv, KrylovScalars* sc,
-                             KrylovWork& W, int iters, cudaStream_t s)
+cudaError_t iterate_resident(const EllMatrix& A, const R* vals, const R* b, double tol, int max_iter,
+                             const int32_t* stop, R* x, R* r, R* rh, R* p, R* v, R* sv, KrylovScalars* sc,
+                             KrylovScalars* host, KrylovWork& W, int iters, cudaStream_t s)
 {
     int dev = 0;
     ResidentPlan P;
     cudaError_t e = device_plan(A.rows, A.width, sizeof(R), &dev, &P);
     if (e != cudaSuccess) return e;
     if (!P.ok || (int64_t)3 * kSums * P.ctas > (int64_t)W.grid * kPartStride) return cudaErrorCooperativeLaunchTooLarge;
-    e = cudaMemsetAsync(W.counters, 0, kCounterWords * sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
-    const ResidentArgs<R> a{A.cols, vals, A.width, A.rows, P.rc, P.x_in_smem ? 1 : 0, x, r, rh, p, v, sv, sc, W.partials,
-                            W.counters + kBarrierFirst, reinterpret_cast<int*>(W.counters + kBarrierError), iters};
+    const ResidentArgs<R> a{A.cols, vals, A.width, A.rows, P.rc, P.x_in_smem ? 1 : 0, x, r, rh, p, v, sv, b, tol,
+                            max_iter, stop, sc, host, W.partials, W.counters + kBarrierFirst,
+                            reinterpret_cast<int*>(W.counters + kBarrierError), iters};
     MHFEM_WIDTH_DISPATCH(A.width, e = (launch_form<R, WW>(P, a, dev, s)));
     return e;
 }
