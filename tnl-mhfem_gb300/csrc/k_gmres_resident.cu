@@ -421,7 +421,7 @@ GmresPlan plan_gmres(int64_t rows, int width, int vectors, int sms, size_t smem_
     auto fill = [&](int64_t ctas) {
         P.ctas = (int)std::max<int64_t>(1, ctas);
         P.rc = (int)((rows + P.ctas - 1) / P.ctas);
-        P.threads = P.rc <= 128 ? 128 : kGmresThreads;
+        P.threads = std::min(kGmresThreads, group_threads(P.rc, kGmresThreads));
         P.smem = sizeof(double) * (size_t)kSums * P.threads +
                  (P.mem ? 0 : (sizeof(double) * (vectors + width) + sizeof(int32_t) * width) * (size_t)P.rc);
         return P.smem <= smem_max;

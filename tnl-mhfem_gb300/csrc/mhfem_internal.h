@@ -229,14 +229,12 @@ void krylov_iterate_fp64(const EllMatrix& A, double* x, KrylovWork& W, int iters
 // Rows up to which GMRES runs resident.
 int64_t krylov_small_rows();
 // Words of KrylovWork::counters: [0] the reductions' ticket, [3] the flag of a
-// resident solve's wait that gave up, then the resident solves' four arrival
-// counters, each on a 128-byte line of its own with the count at the end of
-// the last launch behind it.  Zero before the first launch and after one whose
-// wait gave up.
+// resident solve's wait that gave up, then (on a 128-byte line of its own) the
+// resident solves' arrival count and its value at the end of the last launch.
+// Zero before the first launch and after one whose wait gave up.
 constexpr int kBarrierError = 3;
 constexpr int kBarrierFirst = 32;
-constexpr int kBarrierStride = 32;
-constexpr int kCounterWords = kBarrierFirst + 4 * kBarrierStride;
+constexpr int kCounterWords = kBarrierFirst + 32;
 // Whether a system of this size can run resident on the SMs of the current
 // device (resident.cuh).
 bool krylov_resident_fits(int64_t rows, int width, bool fp32);

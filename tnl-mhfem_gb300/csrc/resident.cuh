@@ -22,8 +22,8 @@
 // chain of dependent FP64 additions, divisions and synchronisations: a warp
 // reduction takes 0.2 us, a division 0.27 us, a grid barrier 1.5 us.  Hence:
 //  - a reduction's sums go to different warps (one per FP64 unit of the SM),
-//    each with its own arrival counter, and no thread fence beyond the
-//    counter's own release and acquire;
+//    with one arrival and one polling thread per CTA and no thread fence beyond
+//    the counter's own release and acquire;
 //  - the scalars take one reciprocal of three dependent operations per
 //    reduction, square roots only near the decisions they belong to;
 //  - the systems of a few thousand rows run in one thread-block cluster: its
@@ -63,7 +63,7 @@ struct ResidentArgs {
     KrylovScalars* sc;
     KrylovScalars* host;    // pinned copy of sc for the host (may be null)
     double* partials;   // [3 reductions][kSums][CTA]
-    unsigned int* bar;  // kSums arrival counters, kBarrierStride words apart
+    unsigned int* bar;  // arrival count, and its value at the last launch's end
     int* bar_err;
     int max_its;
 };
@@ -131,21 +131,27 @@ struct Group {
     double* partials;
     unsigned int* bar;
     int* err;
-    // Arrivals that this thread's counter (its warp's) has seen.  The counts
-    // run on from launch to launch: the word behind a counter holds its value
-    // at the last launch's end.
+    // Arrivals that the counter has seen (in the first warp).  The count runs
+    // on from launch to launch: the word behind it holds its value at the last
+    // launch's end.
     unsigned int target = 0;
 
     __device__ __forceinline__ void begin()
     {
-        const int warp = threadIdx.x >> 5;
-        if (!CL && warp < kSums) target = __ldcg(bar + warp * kBarrierStride + 1);
+        if (!CL && threadIdx.x < 32) target = __ldcg(bar + 1);
     }
     // Call once every CTA has passed the launch's last wait.
     __device__ __forceinline__ void end()
     {
-        const int warp = threadIdx.x >> 5;
-        if (!CL && blockIdx.x == 0 && warp < kSums && (threadIdx.x & 31) == 0) bar[warp * kBarrierStride + 1] = target;
+        if (!CL && blockIdx.x == 0 && threadIdx.x == 0) bar[1] = target;
+    }
+
+    // Barrier of the first NV warps.
+    template <int NV>
+    __device__ __forceinline__ void sum_warps_sync()
+    {
+        if constexpr (NV == 1) __syncwarp();
+        else asm volatile("bar.sync 1, %0;" ::"n"(NV * 32) : "memory");
     }
 
     // tot[q] = the sum of every thread's acc[q]; also a barrier that makes
@@ -188,13 +194,16 @@ struct Group {
             if (warp < NV) {
                 double* mine = partials + (int64_t)(kind * kSums + warp) * nc;
                 const double v = warp_sum(lane_sum(col + warp * T, lane, T));
-                int ok = 1;
-                target += nc;
-                if (lane == 0) {
-                    __stcg(mine + blockIdx.x, v);
-                    ok = arrive_and_wait(bar + warp * kBarrierStride, err, target);
+                if (lane == 0) __stcg(mine + blockIdx.x, v);
+                // one arrival and one polling thread per CTA for all the sums:
+                // more of either slow the counter's line down
+                sum_warps_sync<NV>();
+                if (warp == 0) {
+                    target += nc;
+                    if (lane == 0 && !arrive_and_wait(bar, err, target)) *bad = 1;
                 }
-                ok = __shfl_sync(0xffffffffu, ok, 0);
+                sum_warps_sync<NV>();
+                const bool ok = *(volatile int*)bad == 0;
                 double a[5] = {0, 0, 0, 0, 0};  // at most one CTA per SM: 152 partials in one pass
                 if (ok)
                     for (int b = lane; b < nc; b += 160) {
@@ -205,10 +214,7 @@ struct Group {
                         for (int k = 0; k < 5; ++k) a[k] = b == lane ? w[k] : a[k] + w[k];
                     }
                 const double s = warp_sum(((a[0] + a[1]) + (a[2] + a[3])) + a[4]);
-                if (lane == 0) {
-                    tot[warp] = s;
-                    if (!ok) *bad = 1;
-                }
+                if (lane == 0) tot[warp] = s;
             }
             else
                 side(warp - NV);
@@ -654,6 +660,22 @@ constexpr int64_t kRecompEntries = 1000000;
 // In FP32 (with half the vectors' bytes) 42.8 and 56.4 us at 73 MB.
 constexpr int64_t kStreamedBytes = (int64_t)72 << 20;
 
+// Threads of a CTA with `rc` rows: as few passes over them as `most` threads
+// allow, of equal size, whole warps, and at least one warp per FP64 unit.  A
+// thread more is a value more in every block sum, a pass more another round of
+// gather latency.  Measured per iteration: 326 rows 12.4 us with 352 threads
+// (one pass), 13.8 with 192, 14.0 with 256; 793 rows 15.8 with 288 (three),
+// 17.2 with 512, 19.1 with 256; 1,115 rows 18.8 with 384, 20.1 with 512; above
+// 4,096 rows the streamed ELL words want 512 threads (46.7 us against 49.3 with
+// 384 at 5,116 rows, 25.2 and 27.2 in FP32).
+constexpr int kPassThreads = 384;
+int group_threads(int rc, int most)
+{
+    if (rc > 4096) return kMaxThreads;
+    const int passes = (rc + most - 1) / most, per = (rc + passes - 1) / passes;
+    return std::max(128, (per + 31) / 32 * 32);
+}
+
 struct ResidentPlan {
     bool ok = false, cluster = false, mats = false, recomp = false, x_in_smem = false;
     int ctas = 0, threads = 0, rc = 0;
@@ -668,7 +690,7 @@ ResidentPlan plan_resident(int64_t rows, int width, size_t real, int sms, size_t
         P.ctas = ctas;
         P.rc = (int)((rows + ctas - 1) / ctas);
         P.ctas = (int)((rows + P.rc - 1) / P.rc);  // no empty CTA
-        P.threads = P.rc <= 128 ? 128 : (P.rc <= 512 ? 256 : kMaxThreads);
+        P.threads = group_threads(P.rc, kPassThreads);
         const size_t vectors = 5 + (P.recomp ? 1 : 0) + (P.x_in_smem ? 1 : 0);
         P.smem = sizeof(double) * (size_t)kSums * P.threads + real * vectors * P.rc +
                  (P.mats ? (real + sizeof(int32_t)) * (size_t)width * P.rc : 0);
