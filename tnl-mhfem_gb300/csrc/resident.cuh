@@ -62,7 +62,7 @@ struct ResidentArgs {
     const int32_t* stop;    // with b: non-zero word: end at once with KS_ASSEMBLY (may be null)
     KrylovScalars* sc;
     KrylovScalars* host;    // pinned copy of sc for the host (may be null)
-    double* partials;   // [3 reductions][kSums][CTA]
+    double* partials;   // [4 reductions][kSums][CTA]
     unsigned int* bar;  // arrival count, and its value at the last launch's end
     int* bar_err;
     int max_its;
@@ -223,7 +223,10 @@ struct Group {
         }
     }
 
-    __device__ __forceinline__ bool barrier()
+    __device__ __forceinline__ bool barrier() { return barrier([](int) {}); }
+    // The warps behind the first run side() while it waits.
+    template <typename Side>
+    __device__ __forceinline__ bool barrier(Side&& side)
     {
         if constexpr (CL) {
             cluster_barrier();
@@ -235,6 +238,8 @@ struct Group {
                 target += gridDim.x;
                 if (threadIdx.x == 0 && !arrive_and_wait(bar, err, target)) *bad = 1;
             }
+            else
+                side((int)(threadIdx.x >> 5) - 1);
             __syncthreads();
             return *bad == 0;
         }
@@ -300,6 +305,25 @@ __device__ __forceinline__ void end_of_iteration(KrylovScalars* S, EndLimits* li
         S->rho = rho;
 }
 
+// The same after an iteration that did not sum over r: rho' from phase B's
+// sums, the restart test against the last known ||r||, no convergence test.
+__device__ __forceinline__ void end_unchecked(KrylovScalars* S, const EndLimits* lim, double rho)
+{
+    const double rho2 = rho * rho, bound2 = lim->restart2 * S->rr;
+    S->it += 1;
+    S->restart = !(finite_bits(rho2) && greater_bits(bound2, kTiny) && greater_bits(rho2, bound2)) &&
+                 fabs(rho) <= kRestartEps * sqrt(S->rr) * S->rhnorm;
+    if (!finite_bits(rho)) { S->status = KS_NOTFINITE; S->done = 1; }
+    else if (zero_bits(S->omega) || zero_bits(S->rho)) { S->status = KS_BREAKDOWN; S->done = 1; }
+    if (S->done) S->res = sqrt(S->rr) / S->bnorm;
+    S->rho = rho;
+}
+
+// Iterations between the convergence tests of the streamed forms.  There the
+// FP64 pipe bounds the vector phases, and the two sums over r are two of 26
+// operations per row; a solve takes hundreds of iterations.
+constexpr int kStreamedCheckEvery = 4;
+
 // WW: compile-time ELL width (0: run-time).  MATS: the CTA's ELL words are
 // copied to shared memory once.  CL: one cluster, gathers from the CTAs'
 // shared memory.  RECOMP: phase B forms s at each gathered neighbour from its
@@ -312,8 +336,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
     extern __shared__ double smem[];
     __shared__ KrylovScalars S;
     __shared__ double tot[kSums];
-    __shared__ double s_inv_rv;
-    __shared__ double slots[CL ? 3 * kSums * kMaxCluster : 1];
+    __shared__ double s_inv_rv, s_rho_next;
+    __shared__ double slots[CL ? 4 * kSums * kMaxCluster : 1];
     __shared__ int bad;
     const int T = blockDim.x, rc = g.rc, W = WW > 0 ? WW : g.W;
     const int64_t base = (int64_t)blockIdx.x * rc, rows = g.rows;
@@ -351,7 +375,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
     R* sp = srh + rc;
     R* sv = sp + rc;
     R* st = sv + rc;
-    R* ss = RECOMP ? st + rc : sr;  // without RECOMP s takes r's place
+    R* ss = RECOMP ? st + rc : sr;  // without RECOMP s takes r's place, and the next r that of t
     R* sa = st + (RECOMP ? 2 : 1) * rc;
     R* xp = g.x + base;
     if (g.x_in_smem) {
@@ -520,6 +544,24 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
             if (S.done) break;
         }
         const R alpha = (R)S.alpha;
+        // x += f y over the CTA's rows, in the warps that wait for a barrier
+        // or a reduction (`used` of them do not): two FP64 operations per row
+        // and iteration leave the critical path.  Streamed forms only: with
+        // few rows the waiting reduction needs the FP64 pipe more (49,408 rows
+        // 12.4 us per iteration without, 12.7 with it).
+        auto add_to_x = [&](R f, const R* y, int w, int used) {
+            const int step = T - 32 * used;
+            constexpr int U = WW == 4 ? 4 : 1;  // the wider forms have no registers left for more
+            for (int m0 = w * 32 + (threadIdx.x & 31); m0 < n; m0 += U * step) {
+                R xv[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (m0 + u * step < n) xv[u] = xp[m0 + u * step];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (m0 + u * step < n) xp[m0 + u * step] = fma(f, y[m0 + u * step], xv[u]);
+            }
+        };
         // B. s, t = A s, the four sums -> omega, beta
         {
             R acc[4] = {0, 0, 0, 0};
@@ -547,7 +589,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
                     ss[m] = sv_;
                     __stcg(g.s + base + m, sv_);
                 }
-                if (!G.barrier()) return;
+                if (!G.barrier([&](int w) { if (!MATS) add_to_x(alpha, sp, w, 1); })) return;
                 spmv([&](int m) { return ss[m]; }, [&](uint32_t c) { return g.s[c]; },
                      [&](int m, R y) {
                          st[m] = y;
@@ -563,6 +605,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
                     S.ts = ts;
                     S.tt = tt;
                     S.omega = q;
+                    s_rho_next = fma(-q, tot[3], tot[2]);  // rho' = (rh, s) - omega (rh, t)
                     S.half = 0;
                     if (!finite_bits(ts) || !finite_bits(tt)) {
                         S.status = KS_NOTFINITE;
@@ -573,15 +616,15 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
                     else if (zero_bits(tt)) S.half = 1;
                 }
                 else
-                    // beta = (rho' / rho) (alpha / omega) with alpha = rho / (rh, v) and
-                    // rho' = (rh, s) - omega (rh, t)
+                    // beta = (rho' / rho) (alpha / omega) with alpha = rho / (rh, v)
                     S.beta = fma(tot[2], q, -tot[3]) * s_inv_rv;
             }
             __syncthreads();
             if (S.done) break;
         }
         if (S.half) {
-            for (int m = threadIdx.x; m < n; m += T) xp[m] = fma(alpha, sp[m], xp[m]);
+            if (MATS)
+                for (int m = threadIdx.x; m < n; m += T) xp[m] = fma(alpha, sp[m], xp[m]);
             __syncthreads();
             if (threadIdx.x == 0) {
                 S.snorm = 0;
@@ -593,36 +636,60 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
             __syncthreads();
             break;
         }
-        // C. x, r, p, (r, r), (rh, r) -> convergence, restart
+        // C. r, p (and x, while the sums go round), (r, r), (rh, r) -> convergence, restart
         {
             const R omega = (R)S.omega, beta = (R)S.beta;
+            const bool check = MATS || (S.it + 1) % kStreamedCheckEvery == 0 || k + 1 == g.max_its ||
+                               S.it + 1 >= S.max_iter;
             R acc[2] = {0, 0};
+            R* const rnew = RECOMP ? sr : st;
             for (int m = threadIdx.x; m < n; m += T) {
                 const R sv_ = ss[m], pv = sp[m];
-                xp[m] = fma(omega, sv_, fma(alpha, pv, xp[m]));
+                if (MATS) xp[m] = fma(omega, sv_, fma(alpha, pv, xp[m]));
                 const R rv = fma(-omega, st[m], sv_);
                 const R pn = fma(beta, fma(-omega, sv[m], pv), rv);
-                sr[m] = rv;
+                rnew[m] = rv;
                 sp[m] = pn;
                 if (!CL) {
                     __stcg(g.p + base + m, pn);
                     if (RECOMP) __stcg(g.r + base + m, rv);
                 }
-                acc[0] = fma(rv, rv, acc[0]);
-                acc[1] = fma(srh[m], rv, acc[1]);
+                if (check) {
+                    acc[0] = fma(rv, rv, acc[0]);
+                    acc[1] = fma(srh[m], rv, acc[1]);
+                }
             }
-            if (!G.reduce(acc, 2)) return;
-            if (threadIdx.x == 0) end_of_iteration(&S, &limits, tot[0], tot[1], k + 1 == g.max_its);
+            if (check) {
+                if (!G.reduce(acc, 2, [&](int w) { if (!MATS) add_to_x(omega, ss, w, 2); })) return;
+                if (threadIdx.x == 0) end_of_iteration(&S, &limits, tot[0], tot[1], k + 1 == g.max_its);
+            }
+            else {
+                if (!G.barrier([&](int w) { if (!MATS) add_to_x(omega, ss, w, 1); })) return;
+                if (threadIdx.x == 0) end_unchecked(&S, &limits, s_rho_next);
+            }
+            if constexpr (!RECOMP) {  // r is where t was; the next s takes its place, the next t that of this s
+                st = ss;
+                sr = ss = rnew;
+            }
             __syncthreads();
             if (S.done) break;
-            if (S.restart) {
+            if (S.restart) {  // rh = p = r; rho = (r, r)
+                acc[0] = 0;
                 for (int m = threadIdx.x; m < n; m += T) {
                     const R rv = sr[m];
                     srh[m] = rv;
                     sp[m] = rv;
                     if (!CL) __stcg(g.p + base + m, rv);
+                    acc[0] = fma(rv, rv, acc[0]);
                 }
-                if (!G.barrier()) return;
+                const R sum[1] = {acc[0]};
+                if (!G.reduce(sum, 3)) return;
+                if (threadIdx.x == 0) {
+                    S.rho = S.rr = tot[0];
+                    S.rhnorm = sqrt(tot[0]);
+                    limits = end_limits(S);
+                }
+                __syncthreads();
             }
         }
     }
@@ -803,7 +870,7 @@ cudaError_t iterate_resident(const EllMatrix& A, const R* vals, const R* b, doub
     ResidentPlan P;
     cudaError_t e = device_plan(A.rows, A.width, sizeof(R), &dev, &P);
     if (e != cudaSuccess) return e;
-    if (!P.ok || (int64_t)3 * kSums * P.ctas > (int64_t)W.grid * kPartStride) return cudaErrorCooperativeLaunchTooLarge;
+    if (!P.ok || (int64_t)4 * kSums * P.ctas > (int64_t)W.grid * kPartStride) return cudaErrorCooperativeLaunchTooLarge;
     const ResidentArgs<R> a{A.cols, vals, A.width, A.rows, P.rc, P.x_in_smem ? 1 : 0, x, r, rh, p, v, sv, b, tol,
                             max_iter, stop, sc, host, W.partials, W.counters + kBarrierFirst,
                             reinterpret_cast<int*>(W.counters + kBarrierError), iters};
