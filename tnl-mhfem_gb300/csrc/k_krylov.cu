@@ -364,13 +364,18 @@ __device__ __forceinline__ void stream_groups(int64_t nv, const T* const (&in)[K
     }
 }
 
+// The scalars between the phases are one thread's work in a kernel's tail, 64
+// cycles per FP64 operation: reciprocals of three operations (recip_newton)
+// instead of divisions of nine, tests on bit patterns, no square root outside
+// check iterations.
+
 // alpha = rho / (rh, v)
 __device__ __forceinline__ void scalars_alpha(KrylovScalars* sc, const double (&s)[1])
 {
     sc->rv = s[0];
-    if (!finite(s[0])) { sc->status = KS_NOTFINITE; sc->done = 1; }
-    else if (s[0] == 0) { sc->status = KS_BREAKDOWN; sc->done = 1; }
-    else sc->alpha = sc->rho / s[0];
+    if (!finite_bits(s[0])) { sc->status = KS_NOTFINITE; sc->done = 1; }
+    else if (zero_bits(s[0])) { sc->status = KS_BREAKDOWN; sc->done = 1; }
+    else sc->alpha = sc->rho * recip_newton(s[0]);
 }
 
 // s = r - alpha v
@@ -498,8 +503,8 @@ __device__ __forceinline__ void scalars_omega(KrylovScalars* sc, const double (&
         sc->half = 0;
     sc->ts = sum[0];
     sc->tt = sum[1];
-    if (!finite(sum[0]) || !finite(sum[1])) { sc->status = KS_NOTFINITE; sc->done = 1; }
-    else if (sum[1] == 0) {
+    if (!finite_bits(sum[0]) || !finite_bits(sum[1])) { sc->status = KS_NOTFINITE; sc->done = 1; }
+    else if (zero_bits(sum[1])) {
         if constexpr (CHECK) { sc->status = KS_BREAKDOWN; sc->done = 1; }  // ||s|| >= tol, yet A s = 0
         else {
             // A s = 0 on an iteration that does not form ||s||: the matrix is
@@ -511,7 +516,7 @@ __device__ __forceinline__ void scalars_omega(KrylovScalars* sc, const double (&
             sc->half = 1;
         }
     }
-    else sc->omega = sum[0] / sum[1];
+    else sc->omega = sum[0] * recip_newton(sum[1]);
 }
 
 // half step: x += alpha p
@@ -593,10 +598,14 @@ __device__ __forceinline__ void scalars_beta(KrylovScalars* sc, const double (&s
         if (!finite(sc->res)) { sc->status = KS_NOTFINITE; sc->done = 1; return; }
         if (sc->res < sc->tol) { sc->status = KS_CONVERGED; sc->done = 1; return; }
     }
-    else if (!finite(sum[0])) { sc->status = KS_NOTFINITE; sc->done = 1; return; }
-    if (sc->it >= sc->max_iter) { sc->status = KS_MAXITER; sc->done = 1; }
-    else if (sc->omega == 0 || sc->rho == 0) { sc->status = KS_BREAKDOWN; sc->done = 1; }
-    else if (fabs(sum[0]) <= kRestartEps * sqrt(sc->rr) * sc->rhnorm) {
+    else if (!finite_bits(sum[0])) { sc->status = KS_NOTFINITE; sc->done = 1; return; }
+    const double rho = sc->rho, omega = sc->omega, rr = sc->rr, rhnorm = sc->rhnorm;
+    if (sc->it >= sc->max_iter) { sc->status = KS_MAXITER; sc->done = 1; return; }
+    if (zero_bits(omega) || zero_bits(rho)) { sc->status = KS_BREAKDOWN; sc->done = 1; return; }
+    // |(rh, r)| <= kRestartEps ||r|| ||rh||, by the squares where they decide clearly
+    const double e = kRestartEps * rhnorm, s2 = sum[0] * sum[0], bound2 = (e * e) * rr;
+    const bool above = finite_bits(s2) && greater_bits(bound2, kTiny) && greater_bits(s2, bound2 * (1.0 + 1e-9));
+    if (!above && fabs(sum[0]) <= kRestartEps * sqrt(rr) * rhnorm) {
         // shadow residual (numerically) orthogonal to r: restart with rh = p = r
         // (rho = (r, r) and ||rh|| come from update_p's restart pass)
         sc->restart = 1;
@@ -604,7 +613,7 @@ __device__ __forceinline__ void scalars_beta(KrylovScalars* sc, const double (&s
     }
     else {
         sc->restart = 0;
-        sc->beta = (sum[0] / sc->rho) * (sc->alpha / sc->omega);
+        sc->beta = (sum[0] * recip_newton(rho)) * (sc->alpha * recip_newton(omega));
         sc->rho = sum[0];
     }
 }

@@ -110,61 +110,73 @@ constexpr double kRestartEps = 1e-14;
 // Per-block partial sums: up to kPartStride values per block.
 constexpr int kPartStride = 8;
 
-// FP64 sums: every thread parks its sums in shared memory and warp 0 adds
-// them, each lane the KB/32 values of its column in order, then a shuffle
+// Sum of col[lane], col[lane + 32], ... over KB values and the warp's lanes,
+// in a fixed order (in every lane).
+__device__ __forceinline__ double warp_column_sum(const double* col, int lane)
+{
+    static_assert(KB == 256, "eight values per lane");
+    double v[KB / 32];
+#pragma unroll
+    for (int w = 0; w < KB / 32; ++w) v[w] = col[lane + 32 * w];
+    double s = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
+// FP64 sums: every thread parks its sums in shared memory and warp q adds
+// those of value q, each lane the KB/32 values of its column, then a shuffle
 // tree; that is 12 FP64 additions per sum for the block, against 5 in each
 // of the 8 warps plus 8 in thread 0 for a shuffle tree per warp.  The FP64
 // pipe (about 2 operations per clock per SM on GB300) co-limits the FP64
 // iteration kernels with HBM, and at one wave of CTAs over 3.2M rows those
-// trees were about 12% of their FP64 operations.  FP32 sums keep the
-// per-warp trees (their additions use the FP32 pipe).
+// trees were about 12% of their FP64 operations.  A warp issues one FP64
+// operation per 64 cycles whatever its parallelism, so each sum has a warp
+// (and with it one of the SM's four FP64 units) of its own.  FP32 sums keep
+// the per-warp trees (their additions use the FP32 pipe); the eight warps'
+// sums of every value are then added in FP64 side by side, eight lanes to a
+// value.
 template <typename T, int NV>
 __device__ __forceinline__ void block_reduce_store(T (&acc)[NV], double* partials)
 {
-    static_assert(NV <= kPartStride, "too many partial sums");
+    static_assert(NV <= kPartStride && kPartStride <= KB / 32, "a warp per partial sum");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if constexpr (sizeof(T) == 8) {
         __shared__ double col[NV][KB];
 #pragma unroll
         for (int q = 0; q < NV; ++q) col[q][threadIdx.x] = acc[q];
         __syncthreads();
-        if (warp == 0) {
-#pragma unroll
-            for (int q = 0; q < NV; ++q) {
-                double v = col[q][lane];
-#pragma unroll
-                for (int w = 1; w < KB / 32; ++w) v += col[q][lane + 32 * w];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-                if (lane == 0) partials[(int64_t)blockIdx.x * kPartStride + q] = v;
-            }
+        if (warp < NV) {
+            const double v = warp_column_sum(col[warp], lane);
+            if (lane == 0) partials[(int64_t)blockIdx.x * kPartStride + warp] = v;
         }
     }
     else {
-        __shared__ double sh[KB / 32][kPartStride];
+        static_assert(NV <= 4, "eight lanes per value");
+        __shared__ float sh[kPartStride][KB / 32];
 #pragma unroll
         for (int q = 0; q < NV; ++q) {
             T v = acc[q];
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if (lane == 0) sh[warp][q] = (double)v;
+            if (lane == 0) sh[q][warp] = v;
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
+        if (warp == 0) {
+            const int q = lane / (KB / 32);
+            double v = q < NV ? (double)sh[q][lane % (KB / 32)] : 0.0;
 #pragma unroll
-            for (int q = 0; q < NV; ++q) {
-                double s = 0;
-                for (int w = 0; w < KB / 32; ++w) s += sh[w][q];
-                partials[(int64_t)blockIdx.x * kPartStride + q] = s;
-            }
+            for (int o = KB / 64; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (q < NV && lane % (KB / 32) == 0) partials[(int64_t)blockIdx.x * kPartStride + q] = v;
         }
     }
 }
 
 // Returns true in the last block to finish; that block then sees every
-// partial.  Thread 0 wrote this block's partial, so only thread 0 fences
-// before taking its ticket (the other threads' stores need no ordering: the
-// last block reads partials only).  The counter is reset for the next launch.
+// partial.  The warps that wrote this block's partials did so before the
+// first __syncthreads, after which thread 0 fences and takes its ticket (the
+// other threads' stores need no ordering: the last block reads partials only).
+// The counter is reset for the next launch.
 __device__ __forceinline__ bool ticket_last(uint32_t* counter)
 {
     __shared__ bool last;
@@ -179,17 +191,22 @@ __device__ __forceinline__ bool ticket_last(uint32_t* counter)
     return last;
 }
 
-// Deterministic sum of the partials by the last block (fixed order): every
-// thread issues its (at most four per pass) partial loads together, the warp
-// sums them with shuffles and warp 0 adds the eight warp sums in order.
+// Deterministic sum of the partials by the last block (fixed order), in out[]
+// of thread 0: every thread issues its (at most four per pass) partial loads
+// together, then warp q adds the threads' sums of value q.  Shuffle trees in
+// every warp and a sum over the warps in every thread, as before, kept the
+// FP64 pipe of the one SM that works here busy for 2,600 cycles per value
+// (1.3 us of every reduction's tail), now 600 and one tree.
 template <int NV>
 __device__ __forceinline__ void final_sums(const double* partials, double (&out)[NV])
 {
-    __shared__ double sh[KB / 32][kPartStride];
+    static_assert(NV <= KB / 32, "a warp per value");
+    __shared__ double col[NV][KB];
+    __shared__ double tot[NV];
     double acc[NV];
+    const int nb = (int)gridDim.x;
 #pragma unroll
     for (int q = 0; q < NV; ++q) acc[q] = 0;
-    const int nb = (int)gridDim.x;
     for (int b0 = threadIdx.x; b0 < nb; b0 += 4 * KB) {
         double v[4][NV];
 #pragma unroll
@@ -200,25 +217,22 @@ __device__ __forceinline__ void final_sums(const double* partials, double (&out)
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
+            if (b0 + j * KB < nb) {
 #pragma unroll
-            for (int q = 0; q < NV; ++q) acc[q] += v[j][q];
+                for (int q = 0; q < NV; ++q) acc[q] += v[j][q];
+            }
     }
+#pragma unroll
+    for (int q = 0; q < NV; ++q) col[q][threadIdx.x] = acc[q];
+    __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int q = 0; q < NV; ++q) {
-        double v = acc[q];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) sh[warp][q] = v;
+    if (warp < NV) {
+        const double v = warp_column_sum(col[warp], lane);
+        if (lane == 0) tot[warp] = v;
     }
     __syncthreads();
 #pragma unroll
-    for (int q = 0; q < NV; ++q) {
-        double t = 0;
-#pragma unroll
-        for (int w = 0; w < KB / 32; ++w) t += sh[w][q];
-        out[q] = t;
-    }
+    for (int q = 0; q < NV; ++q) out[q] = tot[q];
 }
 
 // Programmatic dependent launch: the iteration kernels are launched with
@@ -265,6 +279,20 @@ __device__ __forceinline__ T spmv_row(const int32_t* __restrict__ cols, const T*
 }
 
 __device__ __forceinline__ bool finite(double v) { return isfinite(v); }
+
+// Tests on the bit pattern keep comparisons off the FP64 pipe (64 cycles each).
+__device__ __forceinline__ bool finite_bits(double v)
+{
+    return (__double_as_longlong(v) & 0x7ff0000000000000LL) != 0x7ff0000000000000LL;
+}
+__device__ __forceinline__ bool zero_bits(double v) { return (__double_as_longlong(v) << 1) == 0; }
+// a > b for a >= 0, b >= 0 and both finite
+__device__ __forceinline__ bool greater_bits(double a, double b)
+{
+    return __double_as_longlong(a) > __double_as_longlong(b);
+}
+
+constexpr double kTiny = 1e-280;  // squares above this are far from the range's end
 
 // ---- vector access -------------------------------------------------------------
 //

@@ -246,20 +246,6 @@ struct Group {
     }
 };
 
-// Tests on the bit pattern keep comparisons off the FP64 pipe (64 cycles each).
-__device__ __forceinline__ bool finite_bits(double v)
-{
-    return (__double_as_longlong(v) & 0x7ff0000000000000LL) != 0x7ff0000000000000LL;
-}
-__device__ __forceinline__ bool zero_bits(double v) { return (__double_as_longlong(v) << 1) == 0; }
-// a > b for a >= 0, b >= 0 and both finite
-__device__ __forceinline__ bool greater_bits(double a, double b)
-{
-    return __double_as_longlong(a) > __double_as_longlong(b);
-}
-
-constexpr double kTiny = 1e-280;  // squares above this are far from the range's end
-
 // Limits that decide a common iteration's end without a square root or a
 // quotient: (tol ||b||)^2 and (kRestartEps ||rh||)^2, each with a margin far
 // above the rounding of the comparison it stands for.
