@@ -1,9 +1,10 @@
-"""The FP64 BiCGStab resident on the SMs (csrc/k_resident.cu) at the edges of
+"""The FP64 BiCGStab resident on the SMs (csrc/resident.cuh, resident_two.cuh) at the edges of
 its forms, against the oracle: one CTA, clusters of 2 to 16 with a partial
 last block of rows, the largest cluster and the first grid, both sides of the
-size where phase B stops forming the neighbours' s, the sizes where the ELL
-words and then x leave shared memory, and the last resident system and the
-first one above it; run-time and compile-time widths.
+sizes where an iteration goes from two reductions to three and where phase B
+stops forming the neighbours' s, the sizes where the ELL words and then x
+leave shared memory, and the last resident system and the first one above it;
+run-time and compile-time widths.
 
 The bar is the parity tests': both sides solve to 1e-13, the states agree
 within 1e-10.
@@ -26,20 +27,28 @@ SIZES = [
     ("heat2d", 6),           # 120
     ("heat2d", 7),           # 161: a cluster of 2
     ("heat2d", 17),          # 901: 8, the last block partial
-    ("heat2d", 51),          # 7,905: the largest cluster
-    ("heat2d", 53),          # 8,533: the smallest grid
-    ("heat2d", 162),         # 79,056: neighbours' s recomputed
-    ("heat2d", 164),         # 81,016: s published
+    ("heat2d", 36),          # 3,960: the largest cluster
+    ("heat2d", 37),          # 4,181: the smallest grid
+    ("heat2d", 53),          # 8,533
+    ("heat2d", 162),         # 79,056
+    ("heat2d", 203),         # 124,033: two reductions per iteration
+    ("heat2d", 205),         # 126,485: three, the neighbours' s recomputed
+    ("heat2d", 288),         # 249,408
+    ("heat2d", 290),         # 252,880: s published
     ("heat2d", 345),         # 357,765: ELL words streamed
     ("heat2d", 520),         # 812,240: x in memory, the largest resident system
     ("heat2d", 523),         # 821,633: five kernels
     ("diffusion3d", 3),      # width 6: 378
+    ("diffusion3d", 7),      # 4,410
     ("diffusion3d", 13),     # 27,378
+    ("diffusion3d", 19),     # 84,474
     ("diffusion3d", 29),     # 297,714: streamed
     ("diffusion3d_box", 9),  # width 10: 2,430
+    ("diffusion3d_box", 24),  # 43,200
     ("diffusion3d_box", 36),  # 143,856
     ("diffusion3d_box", 50),  # 382,500: streamed
     ("adr2d", 15),           # width 9: 1,410
+    ("adr2d", 60),           # 21,840
     ("adr2d", 120),          # 86,880
     ("adr2d", 240),          # 346,560: streamed
     ("diffusion3d_n2", 6),   # width 13: 5,616
@@ -76,7 +85,7 @@ def test_resident_solve_against_oracle(name, N):
     s.close()
 
 
-@pytest.mark.parametrize("name,N", [("heat2d", 40), ("heat2d", 100), ("diffusion3d", 29)])
+@pytest.mark.parametrize("name,N", [("heat2d", 30), ("heat2d", 40), ("heat2d", 100), ("diffusion3d", 29)])
 def test_resident_solve_continues_after_a_chunk(name, N):
     """A time step 400 times as long takes more iterations than one launch
     runs (256): the solve goes on from the state the launch left, in the
@@ -95,8 +104,9 @@ def test_resident_solve_continues_after_a_chunk(name, N):
 
 @pytest.mark.parametrize("name,N", [
     ("heat2d", 6),            # one CTA
-    ("heat2d", 51),           # the largest cluster
-    ("heat2d", 53),           # the smallest grid
+    ("heat2d", 36),           # the largest cluster
+    ("heat2d", 37),           # the smallest grid
+    ("heat2d", 200),          # 120,400: two reductions per iteration
     ("heat2d", 391),          # 459,425: the ELL words still in shared memory
     ("heat2d", 405),          # 492,885: streamed
     ("diffusion3d", 13),
@@ -125,8 +135,8 @@ def test_resident_inner_solve_against_oracle(name, N):
 @pytest.mark.parametrize("name,N", [
     ("heat2d", 2),             # one CTA, the Krylov space as large as the system
     ("heat2d", 17),            # a cluster, the last block partial
-    ("heat2d", 51),            # the largest cluster
-    ("heat2d", 53),            # the smallest grid
+    ("heat2d", 36),            # the largest cluster
+    ("heat2d", 37),            # the smallest grid
     ("heat2d", 150),           # 67,800: the basis in shared memory
     ("heat2d", 200),           # 120,400: the basis in memory
     ("heat2d", 300),           # 270,600

@@ -13,8 +13,8 @@ bool krylov_resident_fits(int64_t rows, int width, bool fp32)
 cudaError_t krylov_resident_fp64(const EllMatrix& A, const double* b, double tol, int max_iter, const int32_t* stop,
                                  double* x, KrylovWork& W, KrylovScalars* host, int iters, cudaStream_t s)
 {
-    return iterate_resident<double>(A, A.vals, b, tol, max_iter, stop, x, W.r, W.rh, W.p, W.v, W.s, W.sc, host, W,
-                                    iters, s);
+    return iterate_resident<double>(A, A.vals, b, tol, max_iter, stop, x, W.r, W.rh, W.p, W.v, W.s, W.t, W.sc, host,
+                                    W, iters, s);
 }
 
 }  // namespace mhfem

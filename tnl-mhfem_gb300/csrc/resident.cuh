@@ -6,7 +6,8 @@
 // of rows and keeps their Krylov vectors in shared memory for the whole
 // launch (for the smaller systems the rows' ELL words too), so that only
 // what the SpMVs gather goes through memory, and an iteration is three (or
-// four) phases separated by group-wide reductions instead of five kernels:
+// four) phases separated by group-wide reductions instead of five kernels
+// (the smallest systems take resident_two.cuh's form of two):
 //   A. v = A p, (rh, v) -> alpha;
 //   B. s = r - alpha v, t = A s, (t, s), (t, t), (rh, s), (rh, t) -> omega and
 //      beta;
@@ -26,8 +27,9 @@
 //    the counter's own release and acquire;
 //  - the scalars take one reciprocal of three dependent operations per
 //    reduction, square roots only near the decisions they belong to;
-//  - the systems of a few thousand rows run in one thread-block cluster: its
-//    barrier takes 0.5 us and the gathers read the neighbours' shared memory.
+//  - the systems of a few thousand rows run in one thread-block cluster
+//    (resident_two.cuh): its barrier takes 0.5 us and the gathers read the
+//    neighbours' shared memory.
 // Every wait on a grid counter is bounded: a CTA that polls kBarrierPolls
 // times records the failure in *bar_err and returns, and the others then fail
 // their waits too.
@@ -41,12 +43,6 @@
 
 namespace mhfem {
 
-namespace {
-
-constexpr int kMaxThreads = 512;
-constexpr int kSums = 4;          // sums of the widest reduction
-constexpr int kMaxCluster = 16;
-
 template <typename T>
 struct ResidentArgs {
     const int32_t* cols;
@@ -55,7 +51,7 @@ struct ResidentArgs {
     int64_t rows;
     int rc;             // rows per CTA
     int x_in_smem;
-    T *x, *r, *rh, *p, *v, *s;
+    T *x, *r, *rh, *p, *v, *s, *t;
     const T* b;             // right-hand side: the launch begins the solve (r = b - A x); null: it goes on
     double tol;             // with b: the solve's limits
     int max_iter;
@@ -67,6 +63,13 @@ struct ResidentArgs {
     int* bar_err;
     int max_its;
 };
+
+namespace {
+
+constexpr int kMaxThreads = 512;
+constexpr int kPassThreads = 384;  // most threads of a CTA whose rows are few (group_threads)
+constexpr int kSums = 4;          // sums of the widest reduction
+constexpr int kMaxCluster = 16;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -305,55 +308,107 @@ __device__ __forceinline__ void end_unchecked(KrylovScalars* S, const EndLimits*
     S->rho = rho;
 }
 
+// What a launch begins with: the scalars of a new solve (or those the last
+// launch left), nothing else to do if the solve is over.  False when it is.
+template <typename R>
+__device__ __forceinline__ bool begin_resident(const ResidentArgs<R>& g, KrylovScalars* S, EndLimits* limits, int* bad)
+{
+    if (threadIdx.x == 0) {
+        if (g.b) {
+            *S = KrylovScalars{};
+            S->tol = g.tol;
+            S->max_iter = g.max_iter;
+            if (g.stop && *g.stop) {
+                S->status = KS_ASSEMBLY;
+                S->done = 1;
+            }
+        }
+        else {
+            *S = *g.sc;
+            *limits = end_limits(*S);
+        }
+        *bad = 0;
+    }
+    __syncthreads();
+    if (!S->done) return true;  // the same in every CTA
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *g.sc = *S;
+        if (g.host) *g.host = *S;
+    }
+    return false;
+}
+
+// ||r||, ||b|| of a new solve.
+__device__ __forceinline__ void first_residual(KrylovScalars* S, EndLimits* limits, double rr, double bb)
+{
+    const double rn = sqrt(rr), bn = sqrt(bb);
+    S->bnorm = bn == 0 ? 1.0 : bn;
+    S->rho = S->rr = rr;
+    S->rhnorm = rn;
+    S->res = rn / S->bnorm;
+    if (!finite(S->res)) { S->status = KS_NOTFINITE; S->done = 1; }
+    else if (S->res < S->tol) { S->status = KS_CONVERGED; S->done = 1; }
+    *limits = end_limits(*S);
+}
+
+// Two quotients in the first two lanes: omega = ts / tt (and rho' = (rh, s) -
+// omega (rh, t) when rho_next is not null), then beta from tt / ts.
+__device__ __forceinline__ void scalars_omega_beta(KrylovScalars* S, const double* tot, double inv_rv, double* rho_next)
+{
+    const double ts = tot[0], tt = tot[1];
+    const double num = threadIdx.x == 0 ? ts : tt, den = threadIdx.x == 0 ? tt : ts;
+    const double q = num * recip_newton(den);
+    if (threadIdx.x == 0) {
+        S->ts = ts;
+        S->tt = tt;
+        S->omega = q;
+        if (rho_next) *rho_next = fma(-q, tot[3], tot[2]);
+        S->half = 0;
+        if (!finite_bits(ts) || !finite_bits(tt)) {
+            S->status = KS_NOTFINITE;
+            S->done = 1;
+            S->res = sqrt(S->rr) / S->bnorm;
+        }
+        // A s = 0 with a nonsingular matrix: s = 0, and x + alpha p solves the system
+        else if (zero_bits(tt)) S->half = 1;
+    }
+    else
+        // beta = (rho' / rho) (alpha / omega) with alpha = rho / (rh, v)
+        S->beta = fma(tot[2], q, -tot[3]) * inv_rv;
+}
+
+__device__ __forceinline__ void scalars_half_step(KrylovScalars* S)
+{
+    S->snorm = 0;
+    S->res = 0;
+    S->it += 1;
+    S->status = KS_CONVERGED;
+    S->done = 1;
+}
+
 // Iterations between the convergence tests of the streamed forms.  There the
 // FP64 pipe bounds the vector phases, and the two sums over r are two of 26
 // operations per row; a solve takes hundreds of iterations.
 constexpr int kStreamedCheckEvery = 4;
 
 // WW: compile-time ELL width (0: run-time).  MATS: the CTA's ELL words are
-// copied to shared memory once.  CL: one cluster, gathers from the CTAs'
-// shared memory.  RECOMP: phase B forms s at each gathered neighbour from its
+// copied to shared memory once.  RECOMP: phase B forms s at each gathered neighbour from its
 // r and v (W more FP64 operations per row) instead of publishing s behind a
 // barrier of its own.
-template <typename R, int WW, bool MATS, bool CL, bool RECOMP>
+template <typename R, int WW, bool MATS, bool RECOMP>
 __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const ResidentArgs<R> g)
 {
-    static_assert(!CL || (MATS && RECOMP), "the cluster form keeps everything in shared memory");
     extern __shared__ double smem[];
     __shared__ KrylovScalars S;
     __shared__ double tot[kSums];
     __shared__ double s_inv_rv, s_rho_next;
-    __shared__ double slots[CL ? 4 * kSums * kMaxCluster : 1];
     __shared__ int bad;
     const int T = blockDim.x, rc = g.rc, W = WW > 0 ? WW : g.W;
     const int64_t base = (int64_t)blockIdx.x * rc, rows = g.rows;
     const int n = (int)max((int64_t)0, min((int64_t)rc, rows - base));
     __shared__ EndLimits limits;
     const bool first = g.b != nullptr;
-    if (threadIdx.x == 0) {
-        if (first) {
-            S = KrylovScalars{};
-            S.tol = g.tol;
-            S.max_iter = g.max_iter;
-            if (g.stop && *g.stop) {
-                S.status = KS_ASSEMBLY;
-                S.done = 1;
-            }
-        }
-        else {
-            S = *g.sc;
-            limits = end_limits(S);
-        }
-        bad = 0;
-    }
-    __syncthreads();
-    if (S.done) {  // the same in every CTA
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            *g.sc = S;
-            if (g.host) *g.host = S;
-        }
-        return;
-    }
+    if (!begin_resident(g, &S, &limits, &bad)) return;
 
     double* col = smem;
     R* sr = reinterpret_cast<R*>(col + kSums * T);
@@ -384,13 +439,11 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
                 const int64_t o = (int64_t)k * rows + base + m;
                 const uint32_t c = (uint32_t)__ldg(g.cols + o);
                 sa[k * rc + m] = __ldg(g.vals + o);
-                // cluster: the column's address in its owner's copy of sr
-                scol[k * rc + m] = CL ? map_rank(smem_u32(sr + c % rc), c / rc) : c;
+                scol[k * rc + m] = c;
             }
-    Group<CL> G{col, tot, slots, &bad, g.partials, g.bar, g.bar_err};
+    Group<false> G{col, tot, nullptr, &bad, g.partials, g.bar, g.bar_err};
     G.begin();
-    if constexpr (CL) cluster_barrier();  // every CTA's shared memory is set up
-    else __syncthreads();
+    __syncthreads();
 
     // y = self + sum_k a_k gather(c_k) over the CTA's rows; body(m, y).  The
     // streamed form loads the next row's ELL words before the current gathers.
@@ -467,7 +520,6 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
             }
         }
     };
-    const uint32_t off_p = (uint32_t)((char*)sp - (char*)sr), off_v = (uint32_t)((char*)sv - (char*)sr);
 
     if (first) {
         // rh = p = r = b - A x (x gathered from memory), ||r||, ||b||
@@ -482,24 +534,13 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
             sr[m] = rv;
             srh[m] = rv;
             sp[m] = rv;
-            if (!CL) {
-                __stcg(g.p + base + m, rv);
-                if (RECOMP) __stcg(g.r + base + m, rv);
-            }
+            __stcg(g.p + base + m, rv);
+            if (RECOMP) __stcg(g.r + base + m, rv);
             acc[0] = fma(rv, rv, acc[0]);
             acc[1] = fma(bm, bm, acc[1]);
         }
         if (!G.reduce(acc, 2)) return;
-        if (threadIdx.x == 0) {
-            const double rn = sqrt(tot[0]), bn = sqrt(tot[1]);
-            S.bnorm = bn == 0 ? 1.0 : bn;
-            S.rho = S.rr = tot[0];
-            S.rhnorm = rn;
-            S.res = rn / S.bnorm;
-            if (!finite(S.res)) { S.status = KS_NOTFINITE; S.done = 1; }
-            else if (S.res < S.tol) { S.status = KS_CONVERGED; S.done = 1; }
-            limits = end_limits(S);
-        }
+        if (threadIdx.x == 0) first_residual(&S, &limits, tot[0], tot[1]);
         __syncthreads();
     }
 
@@ -508,10 +549,10 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
         {
             R acc[1] = {0};
             spmv([&](int m) { return sp[m]; },
-                 [&](uint32_t c) { return CL ? ld_cluster<R>(c + off_p) : g.p[c]; },
+                 [&](uint32_t c) { return g.p[c]; },
                  [&](int m, R y) {
                      sv[m] = y;
-                     if (RECOMP && !CL) __stcg(g.v + base + m, y);
+                     if (RECOMP) __stcg(g.v + base + m, y);
                      acc[0] = fma(srh[m], y, acc[0]);
                  });
             if (!G.reduce(acc, 0)) return;
@@ -560,10 +601,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
             };
             if constexpr (RECOMP) {
                 spmv([&](int m) { return ss[m] = fma(-alpha, sv[m], sr[m]); },
-                     [&](uint32_t c) {
-                         return CL ? fma(-alpha, ld_cluster<R>(c + off_v), ld_cluster<R>(c))
-                                   : fma(-alpha, g.v[c], g.r[c]);
-                     },
+                     [&](uint32_t c) { return fma(-alpha, g.v[c], g.r[c]); },
                      [&](int m, R y) {
                          st[m] = y;
                          dots(m, ss[m], y);
@@ -583,28 +621,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
                      });
             }
             if (!G.reduce(acc, 1)) return;
-            if (threadIdx.x < 2) {  // two quotients in two lanes: omega = ts / tt, then beta from tt / ts
-                const double ts = tot[0], tt = tot[1];
-                const double num = threadIdx.x == 0 ? ts : tt, den = threadIdx.x == 0 ? tt : ts;
-                const double q = num * recip_newton(den);
-                if (threadIdx.x == 0) {
-                    S.ts = ts;
-                    S.tt = tt;
-                    S.omega = q;
-                    s_rho_next = fma(-q, tot[3], tot[2]);  // rho' = (rh, s) - omega (rh, t)
-                    S.half = 0;
-                    if (!finite_bits(ts) || !finite_bits(tt)) {
-                        S.status = KS_NOTFINITE;
-                        S.done = 1;
-                        S.res = sqrt(S.rr) / S.bnorm;
-                    }
-                    // A s = 0 with a nonsingular matrix: s = 0, and x + alpha p solves the system
-                    else if (zero_bits(tt)) S.half = 1;
-                }
-                else
-                    // beta = (rho' / rho) (alpha / omega) with alpha = rho / (rh, v)
-                    S.beta = fma(tot[2], q, -tot[3]) * s_inv_rv;
-            }
+            if (threadIdx.x < 2) scalars_omega_beta(&S, tot, s_inv_rv, &s_rho_next);
             __syncthreads();
             if (S.done) break;
         }
@@ -612,13 +629,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
             if (MATS)
                 for (int m = threadIdx.x; m < n; m += T) xp[m] = fma(alpha, sp[m], xp[m]);
             __syncthreads();
-            if (threadIdx.x == 0) {
-                S.snorm = 0;
-                S.res = 0;
-                S.it += 1;
-                S.status = KS_CONVERGED;
-                S.done = 1;
-            }
+            if (threadIdx.x == 0) scalars_half_step(&S);
             __syncthreads();
             break;
         }
@@ -636,10 +647,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
                 const R pn = fma(beta, fma(-omega, sv[m], pv), rv);
                 rnew[m] = rv;
                 sp[m] = pn;
-                if (!CL) {
-                    __stcg(g.p + base + m, pn);
-                    if (RECOMP) __stcg(g.r + base + m, rv);
-                }
+                __stcg(g.p + base + m, pn);
+                if (RECOMP) __stcg(g.r + base + m, rv);
                 if (check) {
                     acc[0] = fma(rv, rv, acc[0]);
                     acc[1] = fma(srh[m], rv, acc[1]);
@@ -665,7 +674,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
                     const R rv = sr[m];
                     srh[m] = rv;
                     sp[m] = rv;
-                    if (!CL) __stcg(g.p + base + m, rv);
+                    __stcg(g.p + base + m, rv);
                     acc[0] = fma(rv, rv, acc[0]);
                 }
                 const R sum[1] = {acc[0]};
@@ -690,13 +699,16 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
         *g.sc = S;
         if (g.host) *g.host = S;
     }
-    if constexpr (CL) cluster_barrier();  // no CTA leaves while another may still read its shared memory
 }
 
 // ---- launch shapes ---------------------------------------------------------------
 
-// Rows up to which one cluster takes the system.
-constexpr int64_t kClusterRows = 8192;
+// Rows up to which one cluster takes the system: its barrier costs half of the
+// grid's, its 16 SMs have a tenth of the FP64 units.  Measured per iteration,
+// cluster and grid: 6.5 and 8.7 us at 800 rows (width 4), 7.8 and 8.8 at 3,960,
+// 8.6 and 8.6 at 5,376, 10.6 and 8.7 at 7,905; 9.1 and 10.6 at 2,480 (width 9),
+// 12.0 and 10.9 at 5,520.
+constexpr int64_t kClusterRows = 4096;
 // Off-diagonal entries up to which phase B of the FP64 solve forms the
 // neighbours' s itself: a barrier less against one FP64 operation per entry.
 // Measured per iteration, with and without: 14.97 and 15.84 us at 0.30M
@@ -704,6 +716,14 @@ constexpr int64_t kClusterRows = 8192;
 // 0.79M (width 4), but 22.3 and 21.4 at 1.22M (width 9), 27.1 and 26.4 at
 // 1.44M.  In FP32 the operation costs nothing: always.
 constexpr int64_t kRecompEntries = 1000000;
+
+// Off-diagonal entries up to which the FP64 solve runs with two reductions
+// per iteration (resident_two.cuh).  Measured per iteration against three:
+// 8.6 and 10.1 us at 50,000 entries (width 4), 11.7 and 12.8 at 304,000 (width
+// 6), 13.7 and 14.5 at 432,000, 15.4 and 15.4 at 537,000, but 17.0 and 16.4 at
+// 683,000, 16.9 and 15.8 at 682,000 (width 10).  In FP32 wherever it fits (12.6
+// and 14.7 at 788,000).
+constexpr int64_t kTwoEntries = 500000;
 
 // Matrix bytes up to which the ELL words are streamed from L2 by one CTA per
 // SM (129 MB of L2 also holds the gathered vectors and x).  Measured per
@@ -721,7 +741,6 @@ constexpr int64_t kStreamedBytes = (int64_t)72 << 20;
 // 17.2 with 512, 19.1 with 256; 1,115 rows 18.8 with 384, 20.1 with 512; above
 // 4,096 rows the streamed ELL words want 512 threads (46.7 us against 49.3 with
 // 384 at 5,116 rows, 25.2 and 27.2 in FP32).
-constexpr int kPassThreads = 384;
 int group_threads(int rc, int most)
 {
     if (rc > 4096) return kMaxThreads;
@@ -731,6 +750,7 @@ int group_threads(int rc, int most)
 
 struct ResidentPlan {
     bool ok = false, cluster = false, mats = false, recomp = false, x_in_smem = false;
+    bool two = false;  // resident_two.cuh
     int ctas = 0, threads = 0, rc = 0;
     size_t smem = 0;
 };
@@ -746,20 +766,27 @@ ResidentPlan plan_resident(int64_t rows, int width, size_t real, int sms, size_t
         P.threads = group_threads(P.rc, kPassThreads);
         const size_t vectors = 5 + (P.recomp ? 1 : 0) + (P.x_in_smem ? 1 : 0);
         P.smem = sizeof(double) * (size_t)kSums * P.threads + real * vectors * P.rc +
-                 (P.mats ? (real + sizeof(int32_t)) * (size_t)width * P.rc : 0);
-        return P.smem + 2048 <= smem_max;  // 2 KB for the static shared variables
+                 (P.two    ? (real * (1 + 4 * (size_t)width) + sizeof(int32_t) * width) * P.rc
+                  : P.mats ? (real + sizeof(int32_t)) * (size_t)width * P.rc
+                           : 0);
+        return P.smem + 4096 <= smem_max;  // 4 KB for the static shared variables
     };
-    if (rows <= kClusterRows) {
-        int c = 1;
-        while (c < kMaxCluster && (int64_t)c * 128 < rows) c *= 2;
-        P.cluster = P.mats = P.recomp = P.x_in_smem = true;
-        // every CTA of the cluster is launched, also those left without rows
-        P.ok = fill(c);
-        P.ctas = c;
-        if (P.ok) return P;
-    }
     const int64_t want = (rows + 127) / 128;
     const int ctas = (int)std::min<int64_t>(want, sms);
+    if (real == 4 || rows * width <= kTwoEntries) {
+        // two reductions per iteration, in a cluster or the grid
+        for (bool cluster : {true, false}) {
+            if (cluster && rows > kClusterRows) continue;
+            P = ResidentPlan{};
+            P.two = P.x_in_smem = true;
+            P.cluster = cluster;
+            int c = 1;
+            while (c < kMaxCluster && (int64_t)c * 128 < rows) c *= 2;
+            P.ok = fill(cluster ? c : ctas);
+            if (cluster) P.ctas = c;  // every CTA of the cluster is launched, also those left without rows
+            if (P.ok) return P;
+        }
+    }
     for (int form = 0; form < 3; ++form) {  // ELL words and x in shared memory, x only, neither
         if (form > 0 && (int64_t)(real + 4) * width * rows > kStreamedBytes) return ResidentPlan{};
         P = ResidentPlan{};
@@ -819,21 +846,28 @@ cudaError_t launch_group(void (*kernel)(Args), int ctas, int threads, size_t sme
     return e == cudaErrorInvalidClusterSize ? cudaErrorCooperativeLaunchTooLarge : e;
 }
 
-template <typename R, int WW, bool MATS, bool CL, bool RECOMP>
+template <typename R, int WW, bool MATS, bool RECOMP>
 cudaError_t launch_resident(const ResidentPlan& P, const ResidentArgs<R>& a, int dev, cudaStream_t s)
 {
-    return launch_group<CL>(k_bicgstab_resident<R, WW, MATS, CL, RECOMP>, P.ctas, P.threads, P.smem, a, dev, s);
+    return launch_group<false>(k_bicgstab_resident<R, WW, MATS, RECOMP>, P.ctas, P.threads, P.smem, a, dev, s);
 }
 
 template <typename R, int WW>
 cudaError_t launch_form(const ResidentPlan& P, const ResidentArgs<R>& a, int dev, cudaStream_t s)
 {
-    if (P.cluster) return launch_resident<R, WW, true, true, true>(P, a, dev, s);
-    if (P.mats && P.recomp) return launch_resident<R, WW, true, false, true>(P, a, dev, s);
+    if (P.mats && P.recomp) return launch_resident<R, WW, true, true>(P, a, dev, s);
     if constexpr (sizeof(R) == 8)
-        if (P.mats) return launch_resident<R, WW, true, false, false>(P, a, dev, s);
-    return launch_resident<R, WW, false, false, false>(P, a, dev, s);
+        if (P.mats) return launch_resident<R, WW, true, false>(P, a, dev, s);
+    return launch_resident<R, WW, false, false>(P, a, dev, s);
 }
+
+}  // namespace
+// resident_two.cuh, compiled apart (k_resident_two.cu)
+cudaError_t launch_two(int width, bool cluster, int ctas, int threads, size_t smem, const ResidentArgs<double>& a,
+                       int dev, cudaStream_t s);
+cudaError_t launch_two(int width, bool cluster, int ctas, int threads, size_t smem, const ResidentArgs<float>& a,
+                       int dev, cudaStream_t s);
+namespace {
 
 cudaError_t device_plan(int64_t rows, int width, size_t real, int* dev, ResidentPlan* P)
 {
@@ -849,7 +883,7 @@ cudaError_t device_plan(int64_t rows, int width, size_t real, int* dev, Resident
 // b: begins the solve of A x = b (tol, max_iter, stop); null: goes on with it.
 template <typename R>
 cudaError_t iterate_resident(const EllMatrix& A, const R* vals, const R* b, double tol, int max_iter,
-                             const int32_t* stop, R* x, R* r, R* rh, R* p, R* v, R* sv, KrylovScalars* sc,
+                             const int32_t* stop, R* x, R* r, R* rh, R* p, R* v, R* sv, R* t, KrylovScalars* sc,
                              KrylovScalars* host, KrylovWork& W, int iters, cudaStream_t s)
 {
     int dev = 0;
@@ -857,9 +891,10 @@ cudaError_t iterate_resident(const EllMatrix& A, const R* vals, const R* b, doub
     cudaError_t e = device_plan(A.rows, A.width, sizeof(R), &dev, &P);
     if (e != cudaSuccess) return e;
     if (!P.ok || (int64_t)4 * kSums * P.ctas > (int64_t)W.grid * kPartStride) return cudaErrorCooperativeLaunchTooLarge;
-    const ResidentArgs<R> a{A.cols, vals, A.width, A.rows, P.rc, P.x_in_smem ? 1 : 0, x, r, rh, p, v, sv, b, tol,
+    const ResidentArgs<R> a{A.cols, vals, A.width, A.rows, P.rc, P.x_in_smem ? 1 : 0, x, r, rh, p, v, sv, t, b, tol,
                             max_iter, stop, sc, host, W.partials, W.counters + kBarrierFirst,
                             reinterpret_cast<int*>(W.counters + kBarrierError), iters};
+    if (P.two) return launch_two(A.width, P.cluster, P.ctas, P.threads, P.smem, a, dev, s);
     MHFEM_WIDTH_DISPATCH(A.width, e = (launch_form<R, WW>(P, a, dev, s)));
     return e;
 }
