@@ -115,7 +115,7 @@ typedef struct {
     int32_t check_every;      /* Krylov iterations between host convergence checks (systems
                                  too large for the SMs; an FP64 BiCGStab solve of up to
                                  about 800,000 rows runs resident on them and tests every
-                                 iteration) */
+                                 iteration, above about 340,000 rows every fourth) */
     double  timeout_s;        /* host wall-clock limit of one solve (<= 0: none) */
     int32_t inner_adaptive;   /* mixed form: relax the last sweeps' inner tolerance to what the outer
                                  tolerance still needs (never tighter than inner_tol) */

@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kGmresThreads, 1) k_gmres_resident(const Gmres
     auto sum_dots = [&](int nv, int kind) -> bool {
         __syncthreads();
         double v = 0;
-        if (lane < nv)
+        if (lane < nv && (CL || warp == 0))
             for (int w = 0; w < nw; ++w) v += sh[w][lane];
         const double* src;
         int nc = gridDim.x;

@@ -27,6 +27,7 @@
 //  - decode + loss, the encoder's dZ, Adam: CUDA-core kernels.
 #include <cuda_bf16.h>
 
+#include "fp_convert.h"
 #include "mhfem_internal.h"
 #include "mpnn.h"
 #include "tcgen05.cuh"
@@ -318,55 +319,83 @@ __global__ void __launch_bounds__(NT, TRAIN ? 2 : 3) k_mpnn_layer(const MpnnView
 
 // Training decoder: out = h4 . wd + bd, the loss, dout, dh4 = dout wd and
 // the decoder gradients (one partial per block).
+//
+// Eight lanes share a face's row (16 bytes each, so a warp reads four whole
+// rows and writes four gradients per instruction); the FP64 loss arithmetic of
+// the warp's 32 faces then runs once, a face to a lane.  A row per thread
+// touched 32 rows per instruction and took 104 us at 777,600 faces (43% of
+// HBM for the 392 bytes a face).
 __global__ void __launch_bounds__(256) k_mpnn_decode(const MpnnView V, const double* target, double inv_nt)
 {
-    __shared__ float swd[H];
     __shared__ double red[256 / 32][H + 2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid < H) swd[tid] = V.wd[tid];
-    __syncthreads();
+    const int j = lane & 7, g = lane >> 3;  // columns 8j .. 8j + 7 of the warp's rows 4i + g
+    float wd[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) wd[q] = V.wd[8 * j + q];
     const float bd = V.bd[0];
     double acc_l = 0, acc_db = 0;
-    float acc_w[H];
-#pragma unroll
-    for (int q = 0; q < H; ++q) acc_w[q] = 0.f;
+    float acc_w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     const __nv_bfloat16* h4 = V.h[kMpnnLayers + 1];
-    for (int64_t row = (int64_t)blockIdx.x * 256 + tid; row < V.F; row += (int64_t)gridDim.x * 256) {
-        float hv[H];
-        float out = bd;
+    auto unpack8 = [](const uint4& v, float (&f)[8]) {
+        const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            const uint4 v = *reinterpret_cast<const uint4*>(h4 + row * H + 8 * c);
-            const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+        for (int t = 0; t < 4; ++t) {
+            const float2 p = unpack_bf16(w4[t]);
+            f[2 * t] = p.x;
+            f[2 * t + 1] = p.y;
+        }
+    };
+    for (int64_t base = ((int64_t)blockIdx.x * 8 + warp) * 32; base < V.F; base += (int64_t)gridDim.x * 256) {
+        uint4 v[8];
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                const float2 f = unpack_bf16(w4[t]);
-                hv[8 * c + 2 * t] = f.x;
-                hv[8 * c + 2 * t + 1] = f.y;
+        for (int i = 0; i < 8; ++i) {
+            const int64_t row = base + 4 * i + g;
+            v[i] = row < V.F ? *reinterpret_cast<const uint4*>(h4 + row * H + 8 * j) : make_uint4(0, 0, 0, 0);
+        }
+        float mine = 0;  // the output of face base + 4j + g
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float hv[8], o = 0;
+            unpack8(v[i], hv);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) o = fmaf(hv[q], wd[q], o);
+            o += __shfl_xor_sync(0xffffffffu, o, 4);
+            o += __shfl_xor_sync(0xffffffffu, o, 2);
+            o += __shfl_xor_sync(0xffffffffu, o, 1);
+            if (j == i) mine = o;
+        }
+        const int64_t mrow = base + 4 * j + g;
+        const bool counts = mrow < V.F && V.fixed[mrow] == 0;
+        const double diff = counts ? (double)(bd + mine) - target[mrow] : 0.0;
+        acc_l = fma(diff, diff, acc_l);
+        const float dmine = (float)(2.0 * diff * inv_nt);
+        acc_db += dmine;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float dout = __shfl_sync(0xffffffffu, dmine, (lane & 24) | i);
+            float hv[8], d[8];
+            unpack8(v[i], hv);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                acc_w[q] = fmaf(dout, hv[q], acc_w[q]);
+                d[q] = dout * wd[q];
+            }
+            const int64_t row = base + 4 * i + g;
+            if (row < V.F) {
+                float4* dh = reinterpret_cast<float4*>(V.dh + row * H + 8 * j);
+                dh[0] = make_float4(d[0], d[1], d[2], d[3]);
+                dh[1] = make_float4(d[4], d[5], d[6], d[7]);
             }
         }
-#pragma unroll
-        for (int q = 0; q < H; ++q) out = fmaf(hv[q], swd[q], out);
-        const bool fixed = V.fixed[row] != 0;
-        const double diff = fixed ? 0.0 : ((double)out - target[row]);
-        acc_l += diff * diff;
-        const float dout = (float)(2.0 * diff * inv_nt);
-        acc_db += dout;
-#pragma unroll
-        for (int q = 0; q < H; ++q) acc_w[q] = fmaf(dout, hv[q], acc_w[q]);
-        float* dh = V.dh + row * H;
-#pragma unroll
-        for (int c = 0; c < H / 4; ++c)
-            *reinterpret_cast<float4*>(dh + 4 * c) =
-                make_float4(dout * swd[4 * c], dout * swd[4 * c + 1], dout * swd[4 * c + 2], dout * swd[4 * c + 3]);
     }
     // block reduction of (dwd[64], dbd, loss) into partials[block][66]
 #pragma unroll
-    for (int q = 0; q < H; ++q) {
+    for (int q = 0; q < 8; ++q) {
         float v = acc_w[q];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) red[warp][q] = v;
+        v += __shfl_xor_sync(0xffffffffu, v, 8);
+        v += __shfl_xor_sync(0xffffffffu, v, 16);
+        if (g == 0) red[warp][8 * j + q] = v;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -732,25 +761,54 @@ __global__ void __launch_bounds__(NT) k_mpnn_bwd_dw(const MpnnView V, int layer,
 }
 
 // Sums the per-CTA dW / db partials in a fixed order into the flat gradient.
-__global__ void k_mpnn_reduce_dw(const float* partials, int nparts, int KF, float* gW, float* gb)
+//
+// A block sums 32 values, the partials dealt out to its eight warps; one
+// thread per value was a chain of 304 FP64 additions of 64 cycles (50 us,
+// whatever the mesh), against 5 us of the FP64 pipe over all SMs.
+constexpr int kReduceSlices = 8;
+__global__ void __launch_bounds__(32 * kReduceSlices) k_mpnn_reduce_dw(const float* partials, int nparts, int KF,
+                                                                       float* gW, float* gb)
 {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ double part[kReduceSlices][32];
+    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+    const int idx = blockIdx.x * 32 + lane;
     const int total = KF * H + H;
-    if (idx >= total) return;
-    const int src = idx < KF * H ? idx : TB * H + (idx - KF * H);
     double s = 0;
-    for (int p = 0; p < nparts; ++p) s += partials[(int64_t)p * (TB * H + H) + src];
+    if (idx < total) {
+        const float* src = partials + (idx < KF * H ? idx : TB * H + (idx - KF * H));
+        for (int p0 = slice; p0 < nparts; p0 += 4 * kReduceSlices) {
+            float v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int p = p0 + u * kReduceSlices;
+                v[u] = p < nparts ? src[(int64_t)p * (TB * H + H)] : 0.f;
+            }
+            s += (f32_to_f64(v[0]) + f32_to_f64(v[1])) + (f32_to_f64(v[2]) + f32_to_f64(v[3]));
+        }
+    }
+    part[slice][lane] = s;
+    __syncthreads();
+    if (slice != 0 || idx >= total) return;
+    for (int w = 1; w < kReduceSlices; ++w) s += part[w][lane];
     if (idx < KF * H) gW[idx] = (float)s;
     else gb[idx - KF * H] = (float)s;
 }
 
-__global__ void k_mpnn_reduce_dec(const double* partials, int nparts, float* gwd, float* gbd, double* loss,
-                                  double inv_nt)
+// A block per value (one block for all of them took 55 us, one chain of 608
+// FP64 additions each).
+__global__ void __launch_bounds__(128) k_mpnn_reduce_dec(const double* partials, int nparts, float* gwd, float* gbd,
+                                                         double* loss, double inv_nt)
 {
-    const int idx = threadIdx.x;
-    if (idx >= H + 2) return;
+    __shared__ double part[4];
+    const int idx = blockIdx.x, lane = threadIdx.x & 31;
     double s = 0;
-    for (int p = 0; p < nparts; ++p) s += partials[(int64_t)p * (H + 2) + idx];
+    for (int p = threadIdx.x; p < nparts; p += 128) s += partials[(int64_t)p * (H + 2) + idx];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    s = (part[0] + part[1]) + (part[2] + part[3]);
     if (idx < H) gwd[idx] = (float)s;
     else if (idx == H) gbd[0] = (float)s;
     else *loss = s * inv_nt;  // mean over the training faces
@@ -883,7 +941,7 @@ void mpnn_backward(const MpnnView& V, const double* target, double inv_nt, MpnnG
 {
     const int gdec = mpnn_grid(V.F);
     k_mpnn_decode<<<gdec, 256, 0, s>>>(V, target, inv_nt);
-    k_mpnn_reduce_dec<<<1, 128, 0, s>>>(V.dec_partials, gdec, G.g + G.off_wd, G.g + G.off_bd, G.loss, inv_nt);
+    k_mpnn_reduce_dec<<<H + 2, 128, 0, s>>>(V.dec_partials, gdec, G.g + G.off_wd, G.g + G.off_bd, G.loss, inv_nt);
     const int smdx = smem_req(kDxSmem);
     const int smdw = smem_req(kDwSmem);
     set_smem(k_mpnn_bwd_dx, smdx);
@@ -897,13 +955,13 @@ void mpnn_backward(const MpnnView& V, const double* target, double inv_nt, MpnnG
     for (int l = kMpnnLayers; l >= 1; --l) {
         k_mpnn_bwd_dx<<<gdx, NT, smdx, s>>>(V, l);
         k_mpnn_bwd_dw<128><<<gdw, NT, smdw, s>>>(V, l, G.partials);
-        k_mpnn_reduce_dw<<<(2 * H * H + H + 255) / 256, 256, 0, s>>>(G.partials, gdw, 2 * H, G.g + G.off_W[l],
-                                                                      G.g + G.off_b[l]);
+        k_mpnn_reduce_dw<<<(2 * H * H + H + 31) / 32, 32 * kReduceSlices, 0, s>>>(G.partials, gdw, 2 * H,
+                                                                                  G.g + G.off_W[l], G.g + G.off_b[l]);
     }
     k_mpnn_dz0<<<(unsigned)((V.F * (H / 8) + 255) / 256), 256, 0, s>>>(V);
     k_mpnn_bwd_dw<16><<<gdw0, NT, smdw, s>>>(V, 0, G.partials);
-    k_mpnn_reduce_dw<<<(16 * H + H + 255) / 256, 256, 0, s>>>(G.partials, gdw0, 16, G.g + G.off_W[0],
-                                                              G.g + G.off_b[0]);
+    k_mpnn_reduce_dw<<<(16 * H + H + 31) / 32, 32 * kReduceSlices, 0, s>>>(G.partials, gdw0, 16, G.g + G.off_W[0],
+                                                                           G.g + G.off_b[0]);
 }
 
 void mpnn_adam(float* params, const float* grads, float* m1, float* m2, int n, float lr, int t, cudaStream_t s)
