@@ -50,7 +50,6 @@ struct ResidentArgs {
     int W;
     int64_t rows;
     int rc;             // rows per CTA
-    int x_in_smem;
     T *x, *r, *rh, *p, *v, *s, *t;
     const T* b;             // right-hand side: the launch begins the solve (r = b - A x); null: it goes on
     double tol;             // with b: the solve's limits
@@ -394,8 +393,8 @@ constexpr int kStreamedCheckEvery = 4;
 // WW: compile-time ELL width (0: run-time).  MATS: the CTA's ELL words are
 // copied to shared memory once.  RECOMP: phase B forms s at each gathered neighbour from its
 // r and v (W more FP64 operations per row) instead of publishing s behind a
-// barrier of its own.
-template <typename R, int WW, bool MATS, bool RECOMP>
+// barrier of its own.  XS: x in shared memory.
+template <typename R, int WW, bool MATS, bool RECOMP, bool XS>
 __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const ResidentArgs<R> g)
 {
     extern __shared__ double smem[];
@@ -418,11 +417,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
     R* st = sv + rc;
     R* ss = RECOMP ? st + rc : sr;  // without RECOMP s takes r's place, and the next r that of t
     R* sa = st + (RECOMP ? 2 : 1) * rc;
-    R* xp = g.x + base;
-    if (g.x_in_smem) {
-        xp = sa;
-        sa += rc;
-    }
+    R* const xp = XS ? sa : g.x + base;
+    if (XS) sa += rc;
     uint32_t* scol = reinterpret_cast<uint32_t*>(sa + (int64_t)(MATS ? W : 0) * rc);
 
     for (int m = threadIdx.x; m < n; m += T) {
@@ -431,7 +427,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
             srh[m] = __ldcg(g.rh + base + m);
             sp[m] = __ldcg(g.p + base + m);
         }
-        if (g.x_in_smem) xp[m] = g.x[base + m];
+        if (XS) xp[m] = g.x[base + m];
     }
     if constexpr (MATS)
         for (int k = 0; k < W; ++k)
@@ -575,10 +571,14 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
         // or a reduction (`used` of them do not): two FP64 operations per row
         // and iteration leave the critical path.  Streamed forms only: with
         // few rows the waiting reduction needs the FP64 pipe more (49,408 rows
-        // 12.4 us per iteration without, 12.7 with it).
+        // 12.4 us per iteration without, 12.7 with it).  With x in memory only
+        // at width 4, where registers are left to load four rows together: the
+        // wait does not cover a load per pass (1,515,000 rows in FP32, width 6:
+        // 42.8 us without, 53.8 with it).
+        constexpr bool side_x = !MATS && (XS || WW == 4);
         auto add_to_x = [&](R f, const R* y, int w, int used) {
             const int step = T - 32 * used;
-            constexpr int U = WW == 4 ? 4 : 1;  // the wider forms have no registers left for more
+            constexpr int U = WW == 4 ? 4 : 1;
             for (int m0 = w * 32 + (threadIdx.x & 31); m0 < n; m0 += U * step) {
                 R xv[U];
 #pragma unroll
@@ -613,7 +613,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
                     ss[m] = sv_;
                     __stcg(g.s + base + m, sv_);
                 }
-                if (!G.barrier([&](int w) { if (!MATS) add_to_x(alpha, sp, w, 1); })) return;
+                if (!G.barrier([&](int w) { if (side_x) add_to_x(alpha, sp, w, 1); })) return;
                 spmv([&](int m) { return ss[m]; }, [&](uint32_t c) { return g.s[c]; },
                      [&](int m, R y) {
                          st[m] = y;
@@ -626,7 +626,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
             if (S.done) break;
         }
         if (S.half) {
-            if (MATS)
+            if (!side_x)
                 for (int m = threadIdx.x; m < n; m += T) xp[m] = fma(alpha, sp[m], xp[m]);
             __syncthreads();
             if (threadIdx.x == 0) scalars_half_step(&S);
@@ -642,7 +642,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
             R* const rnew = RECOMP ? sr : st;
             for (int m = threadIdx.x; m < n; m += T) {
                 const R sv_ = ss[m], pv = sp[m];
-                if (MATS) xp[m] = fma(omega, sv_, fma(alpha, pv, xp[m]));
+                if (!side_x) xp[m] = fma(omega, sv_, fma(alpha, pv, xp[m]));
                 const R rv = fma(-omega, st[m], sv_);
                 const R pn = fma(beta, fma(-omega, sv[m], pv), rv);
                 rnew[m] = rv;
@@ -655,11 +655,11 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
                 }
             }
             if (check) {
-                if (!G.reduce(acc, 2, [&](int w) { if (!MATS) add_to_x(omega, ss, w, 2); })) return;
+                if (!G.reduce(acc, 2, [&](int w) { if (side_x) add_to_x(omega, ss, w, 2); })) return;
                 if (threadIdx.x == 0) end_of_iteration(&S, &limits, tot[0], tot[1], k + 1 == g.max_its);
             }
             else {
-                if (!G.barrier([&](int w) { if (!MATS) add_to_x(omega, ss, w, 1); })) return;
+                if (!G.barrier([&](int w) { if (side_x) add_to_x(omega, ss, w, 1); })) return;
                 if (threadIdx.x == 0) end_unchecked(&S, &limits, s_rho_next);
             }
             if constexpr (!RECOMP) {  // r is where t was; the next s takes its place, the next t that of this s
@@ -689,7 +689,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
         }
     }
     for (int m = threadIdx.x; m < n; m += T) {
-        if (g.x_in_smem) g.x[base + m] = xp[m];
+        if (XS) g.x[base + m] = xp[m];
         g.r[base + m] = sr[m];
         g.rh[base + m] = srh[m];
         g.p[base + m] = sp[m];
@@ -846,19 +846,20 @@ cudaError_t launch_group(void (*kernel)(Args), int ctas, int threads, size_t sme
     return e == cudaErrorInvalidClusterSize ? cudaErrorCooperativeLaunchTooLarge : e;
 }
 
-template <typename R, int WW, bool MATS, bool RECOMP>
+template <typename R, int WW, bool MATS, bool RECOMP, bool XS>
 cudaError_t launch_resident(const ResidentPlan& P, const ResidentArgs<R>& a, int dev, cudaStream_t s)
 {
-    return launch_group<false>(k_bicgstab_resident<R, WW, MATS, RECOMP>, P.ctas, P.threads, P.smem, a, dev, s);
+    return launch_group<false>(k_bicgstab_resident<R, WW, MATS, RECOMP, XS>, P.ctas, P.threads, P.smem, a, dev, s);
 }
 
 template <typename R, int WW>
 cudaError_t launch_form(const ResidentPlan& P, const ResidentArgs<R>& a, int dev, cudaStream_t s)
 {
-    if (P.mats && P.recomp) return launch_resident<R, WW, true, true>(P, a, dev, s);
+    if (P.mats && P.recomp) return launch_resident<R, WW, true, true, true>(P, a, dev, s);
     if constexpr (sizeof(R) == 8)
-        if (P.mats) return launch_resident<R, WW, true, false>(P, a, dev, s);
-    return launch_resident<R, WW, false, false>(P, a, dev, s);
+        if (P.mats) return launch_resident<R, WW, true, false, true>(P, a, dev, s);
+    if (P.x_in_smem) return launch_resident<R, WW, false, false, true>(P, a, dev, s);
+    return launch_resident<R, WW, false, false, false>(P, a, dev, s);
 }
 
 }  // namespace
@@ -891,7 +892,7 @@ cudaError_t iterate_resident(const EllMatrix& A, const R* vals, const R* b, doub
     cudaError_t e = device_plan(A.rows, A.width, sizeof(R), &dev, &P);
     if (e != cudaSuccess) return e;
     if (!P.ok || (int64_t)4 * kSums * P.ctas > (int64_t)W.grid * kPartStride) return cudaErrorCooperativeLaunchTooLarge;
-    const ResidentArgs<R> a{A.cols, vals, A.width, A.rows, P.rc, P.x_in_smem ? 1 : 0, x, r, rh, p, v, sv, t, b, tol,
+    const ResidentArgs<R> a{A.cols, vals, A.width, A.rows, P.rc, x, r, rh, p, v, sv, t, b, tol,
                             max_iter, stop, sc, host, W.partials, W.counters + kBarrierFirst,
                             reinterpret_cast<int*>(W.counters + kBarrierError), iters};
     if (P.two) return launch_two(A.width, P.cluster, P.ctas, P.threads, P.smem, a, dev, s);
