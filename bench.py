@@ -76,7 +76,7 @@ def parse_args():
                     help="only the warm-up and timed steps (for an ncu launch list)")
     ap.add_argument("--profile-form", choices=["fp64", "mixed", "learned", "box", "gmres", "heat2d"], default="fp64",
                     help="form used by --profile-run (learned: --learned-train training steps first; heat2d: "
-                         "the FP64 form on the 128^2 heat-equation workload, a small-system solve)")
+                         "the FP64 form on the 128^2 heat-equation workload, a resident solve)")
     return ap.parse_args()
 
 
