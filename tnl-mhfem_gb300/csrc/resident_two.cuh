@@ -30,6 +30,7 @@ __global__ void __launch_bounds__(kPassThreads, 1) k_bicgstab_two(const Resident
     __shared__ EndLimits limits;
     __shared__ double tot[kSums];
     __shared__ double s_inv_rv;
+    __shared__ int s_rv_status;  // KS_RUNNING, or why (rh, v) ends the solve
     __shared__ double slots[CL ? 4 * kSums * kMaxCluster : 1];
     __shared__ int bad;
     const int T = blockDim.x, rc = g.rc, W = WW > 0 ? WW : g.W;
@@ -153,19 +154,29 @@ __global__ void __launch_bounds__(kPassThreads, 1) k_bicgstab_two(const Resident
                 acc[2] = fma(h, r, acc[2]);
             }
             if (!G.reduce(acc, 0)) return;
+            // the tests on the finished iteration and alpha side by side: a
+            // thread's FP64 operations take 64 cycles each
+            const double rho = load ? S.rho : tot[2];
             if (threadIdx.x == 0) {
-                if (!load) end_of_iteration(&S, &limits, tot[1], tot[2], false);
+                if (!load) end_of_iteration(&S, &limits, tot[1], rho, false);
+            }
+            else if (threadIdx.x == 32) {
                 const double rv = tot[0], inv = recip_newton(rv);
                 S.rv = rv;
-                S.alpha = S.rho * inv;
+                S.alpha = rho * inv;
                 s_inv_rv = inv;
-                if (!S.done && !S.restart && (!finite_bits(rv) || zero_bits(rv))) {
-                    S.status = finite_bits(rv) ? KS_BREAKDOWN : KS_NOTFINITE;
+                s_rv_status = !finite_bits(rv) ? KS_NOTFINITE : zero_bits(rv) ? KS_BREAKDOWN : KS_RUNNING;
+            }
+            __syncthreads();
+            if (s_rv_status != KS_RUNNING) {
+                __syncthreads();
+                if (threadIdx.x == 0 && !S.done && !S.restart) {
+                    S.status = s_rv_status;
                     S.done = 1;
                     S.res = sqrt(S.rr) / S.bnorm;
                 }
+                __syncthreads();
             }
-            __syncthreads();
             if (S.done) break;
             if (S.restart) {  // rh = p = r, and phase A again
                 for (int m = threadIdx.x; m < n; m += T) {
