@@ -350,7 +350,7 @@ __device__ __forceinline__ void first_residual(KrylovScalars* S, EndLimits* limi
     *limits = end_limits(*S);
 }
 
-// Two quotients in the first two lanes: omega = ts / tt (and rho' = (rh, s) -
+// Two quotients in threads 0 and 32, side by side: omega = ts / tt (and rho' = (rh, s) -
 // omega (rh, t) when rho_next is not null), then beta from tt / ts.
 __device__ __forceinline__ void scalars_omega_beta(KrylovScalars* S, const double* tot, double inv_rv, double* rho_next)
 {
@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
                      });
             }
             if (!G.reduce(acc, 1)) return;
-            if (threadIdx.x < 2) scalars_omega_beta(&S, tot, s_inv_rv, &s_rho_next);
+            if (threadIdx.x == 0 || threadIdx.x == 32) scalars_omega_beta(&S, tot, s_inv_rv, &s_rho_next);
             __syncthreads();
             if (S.done) break;
         }

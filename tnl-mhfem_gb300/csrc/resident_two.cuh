@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(kPassThreads, 1) k_bicgstab_two(const Resident
                 acc[3] = fma(h, y, acc[3]);
             }
             if (!G.reduce(acc, 1)) return;
-            if (threadIdx.x < 2) scalars_omega_beta(&S, tot, s_inv_rv, nullptr);
+            if (threadIdx.x == 0 || threadIdx.x == 32) scalars_omega_beta(&S, tot, s_inv_rv, nullptr);
             __syncthreads();
             if (S.done) break;
         }
