@@ -358,6 +358,14 @@ mhfem_status mhfem_time_kernel(mhfem_t h, int32_t kernel, int32_t reps, double* 
 mhfem_status mhfem_check_grid_barrier(int32_t device, int32_t ctas, int32_t skip_cta, int32_t max_polls,
                                       int32_t* ctas_passed, int32_t* ctas_gave_up, int32_t* failure_flag);
 
+/* Check of the failure report of the resident solves: from now on CTA `cta`
+ * of their grid launches (negative: none, the default) gives up each of its
+ * waits at once, as a CTA does whose wait ran out.  A solve with such a launch
+ * returns MHFEM_ERR_CUDA, whichever wait it was, and the next one (with -1)
+ * works again.  Launches of fewer CTAs, one-cluster launches (up to 4,096
+ * rows) and the five-kernel iteration have no such wait. */
+mhfem_status mhfem_check_wait_report(mhfem_t h, int32_t cta);
+
 /* ---- learned warm start (MHFEM_FORM_LEARNED) ----------------------------
  * No counterpart in the reference: a message-passing network over the face
  * adjacency graph (3 layers, hidden width 64, BF16 weights, FP32

@@ -243,7 +243,11 @@ mhfem_status mhfem_create(const mhfem_desc* desc, mhfem_t* out)
     for (auto& e : h->ev) ok = ok && cudaEventCreate(&e) == cudaSuccess;
     ok = ok && cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, desc->device) == cudaSuccess;
     ok = ok && cudaMallocHost((void**)&h->W.host_sc, sizeof(KrylovScalars) * 2) == cudaSuccess;
-    ok = ok && cudaMallocHost((void**)&h->host_err, sizeof(int32_t)) == cudaSuccess;
+    ok = ok && cudaMallocHost((void**)&h->host_err, sizeof(int32_t) * 2) == cudaSuccess;
+    if (ok) {
+        h->W.host_wait = h->host_err + 1;
+        *h->W.host_wait = 0;
+    }
     if (!ok) {
         cudaGetLastError();
         mhfem_destroy(h);  // releases whatever was created
@@ -301,9 +305,11 @@ mhfem_status mhfem_set_mesh(mhfem_t h, int64_t V, const double* coords, int64_t 
     h->tags = nullptr; h->bvalues = h->bdirichlet = nullptr;
     h->Z_iF = h->Z_iK = h->v_iKe = h->m_upw = h->Z_upw = h->b = h->R_ijKe = h->R_iK = h->rec = nullptr;
     h->A = EllMatrix(); h->amap = AssemblyMap(); h->rhs = nullptr; h->err_flags = nullptr;
-    KrylovScalars* keep = h->W.host_sc;
+    const KrylovWork keep = h->W;
     h->W = KrylovWork();
-    h->W.host_sc = keep;
+    h->W.host_sc = keep.host_sc;
+    h->W.host_wait = keep.host_wait;
+    h->W.give_up = keep.give_up;
     GmresCtl* keep_gm = h->G.host;
     h->G = GmresWork();
     h->G.host = keep_gm;
@@ -654,9 +660,14 @@ mhfem_status assembly_failed(mhfem_t h)
     return fail(h, MHFEM_ERR_NONPOSITIVE_DIAGONAL, "the diagonal matrix element is not positive");
 }
 
-// A resident launch wrote no result: a wait between its CTAs gave up.
+// Whether a wait between the CTAs of the last resident launch gave up (the
+// stream has been waited for): the launch wrote no result, or the first CTA
+// wrote one although another CTA gave up.
+bool wait_failed(mhfem_t h, int32_t status) { return status == KS_PENDING || *h->W.host_wait != 0; }
+
 mhfem_status wait_gave_up(mhfem_t h, const char* what)
 {
+    *h->W.host_wait = 0;
     CK(cudaMemsetAsync(h->W.counters, 0, kCounterWords * sizeof(uint32_t), h->stream));
     return fail(h, MHFEM_ERR_CUDA, "%s: a grid barrier wait gave up", what);
 }
@@ -726,7 +737,7 @@ mhfem_status run_gmres(mhfem_t h, double tol, int max_iter, const int32_t* stop,
             CK(e);
             h->launches += 1;
             CK(cudaStreamSynchronize(h->stream));
-            if (G.host->status == KS_PENDING) return wait_gave_up(h, "GMRES (resident)");
+            if (wait_failed(h, G.host->status)) return wait_gave_up(h, "GMRES (resident)");
             if (G.host->done) break;
             if (h->opts.timeout_s > 0 && elapsed_s(t0) > h->opts.timeout_s)
                 return fail(h, MHFEM_ERR_TIMEOUT, "Krylov solve exceeded %.1f s", h->opts.timeout_s);
@@ -807,7 +818,7 @@ mhfem_status mhfem::run_fp64(mhfem_t h, double tol, int max_iter, int* iters, do
             CK(e);
             h->launches += 1;
             CK(cudaStreamSynchronize(h->stream));
-            if (h->W.host_sc->status == KS_PENDING) return wait_gave_up(h, "FP64 BiCGStab (resident)");
+            if (wait_failed(h, h->W.host_sc->status)) return wait_gave_up(h, "FP64 BiCGStab (resident)");
             if (h->W.host_sc->done) {
                 *iters = h->W.host_sc->it;
                 *res = h->W.host_sc->res;
@@ -879,7 +890,7 @@ mhfem_status mhfem::run_mixed(mhfem_t h, int* iters, int* sweeps, double* res, c
             return status_from_krylov(h, outer, "mixed-precision refinement");
         }
         for (bool ran = resident; !h->W.host_sc[1].done; ran = true) {
-            if (resident && h->W.host_sc[1].status == KS_PENDING)
+            if (resident && wait_failed(h, h->W.host_sc[1].status))
                 return wait_gave_up(h, "FP32 BiCGStab (resident)");
             if (ran && h->opts.timeout_s > 0 && elapsed_s(t0) > h->opts.timeout_s)
                 return fail(h, MHFEM_ERR_TIMEOUT, "mixed solve exceeded %.1f s", h->opts.timeout_s);
@@ -897,7 +908,7 @@ mhfem_status mhfem::run_mixed(mhfem_t h, int* iters, int* sweeps, double* res, c
             }
             CK(cudaStreamSynchronize(h->stream));
         }
-        if (resident && h->W.host_sc[1].status == KS_PENDING) return wait_gave_up(h, "FP32 BiCGStab (resident)");
+        if (resident && wait_failed(h, h->W.host_sc[1].status)) return wait_gave_up(h, "FP32 BiCGStab (resident)");
         const KrylovScalars inner = h->W.host_sc[1];
         total_inner += inner.it;
         if (inner.status == KS_NOTFINITE)
@@ -1191,6 +1202,13 @@ mhfem_status mhfem_check_grid_barrier(int32_t device, int32_t ctas, int32_t skip
     *ctas_passed = passed;
     *ctas_gave_up = gave_up;
     *failure_flag = flag;
+    return MHFEM_OK;
+}
+
+mhfem_status mhfem_check_wait_report(mhfem_t h, int32_t cta)
+{
+    if (!h) return MHFEM_ERR_INVALID_ARGUMENT;
+    h->W.give_up = cta < 0 ? -1 : cta;
     return MHFEM_OK;
 }
 

@@ -60,7 +60,7 @@ struct mhfem_solver_s {
     mhfem::AssemblyMap amap;
     double* rhs = nullptr;
     int32_t* err_flags = nullptr;
-    int32_t* host_err = nullptr;
+    int32_t* host_err = nullptr;     // pinned: the assembly's error word; the word behind it is W.host_wait
     mhfem::KrylovWork W;
     mhfem::GmresWork G;
 

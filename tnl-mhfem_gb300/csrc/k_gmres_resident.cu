@@ -56,6 +56,8 @@ struct GmresArgs {
     double* partials;
     unsigned int* bar;
     int* bar_err;
+    int* host_wait;     // as ResidentArgs'
+    int give_up;
     int max_its;
 };
 
@@ -128,7 +130,7 @@ __global__ void __launch_bounds__(kGmresThreads, 1) k_gmres_resident(const Gmres
                 scol[k * rc + m] = CL ? map_rank(smem_u32(su + c % rc), c / rc) : c;
             }
     }
-    Group<CL> G{col, tot, slots, &bad, g.partials, g.bar, g.bar_err};
+    Group<CL> G{col, tot, slots, &bad, g.partials, g.bar, g.bar_err, g.host_wait, wait_polls(g.give_up)};
     G.begin();
     if constexpr (CL) cluster_barrier();
     else __syncthreads();
@@ -158,7 +160,7 @@ __global__ void __launch_bounds__(kGmresThreads, 1) k_gmres_resident(const Gmres
                 if (lane < nv) __stcg(mine + blockIdx.x * kDots + lane, v);
                 __syncwarp();
                 G.target += nc;
-                if (lane == 0 && !arrive_and_wait(g.bar, g.bar_err, G.target)) bad = 1;
+                if (lane == 0) G.wait();
             }
             __syncthreads();
             if (bad) return false;
@@ -471,7 +473,8 @@ cudaError_t gmres_resident(const EllMatrix& A, const double* b, double* x, Gmres
         (int64_t)2 * P.ctas * kDots > (int64_t)krylov_grid() * kGmStride)
         return cudaErrorCooperativeLaunchTooLarge;
     const GmresArgs a{A.cols, A.vals, A.width, A.rows, P.rc, reorth ? 1 : 0, G.m + 1, b, x, G.U, G.st, G.host, G.partials,
-                      W.partials, W.counters + kBarrierFirst, reinterpret_cast<int*>(W.counters + kBarrierError), iters};
+                      W.partials, W.counters + kBarrierFirst, reinterpret_cast<int*>(W.counters + kBarrierError),
+                      W.host_wait, W.give_up, iters};
     MHFEM_WIDTH_DISPATCH(A.width, e = launch_gmres_form<WW>(P, a, dev, s));
     return e;
 }

@@ -352,7 +352,8 @@ static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 //
 // Every barrier wait is bounded: a CTA that polls kBarrierPolls times
 // records the failure in *bar_err and returns, and the others then fail
-// their waits too.
+// their next waits.  They need not all fail: the CTA that gives up has arrived,
+// so the others may still pass that wait, and the launch's last one.
 
 constexpr unsigned int kBarrierPolls = 1u << 22;  // seconds, far beyond any barrier of a working launch
 
@@ -364,8 +365,8 @@ __device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int* p)
 }
 
 // Adds one arrival to a grid counter (release) and waits until it reaches
-// `target` (acquire; the count starts at 0 for a launch and grows by one per
-// arrival); one thread.  False when the wait gave up.  The counter's own
+// `target` (acquire; the count grows by one per arrival); one thread.  False
+// when the wait gave up (with max_polls 0: always).  The counter's own
 // release and acquire order the CTA's writes before the arrival (behind a
 // __syncthreads) and its reads after the wait, with no thread fence: 1.5
 // instead of 1.9 us for a barrier over 152 CTAs.
@@ -374,7 +375,7 @@ __device__ __forceinline__ bool arrive_and_wait(unsigned int* count, int* err, u
 {
     asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(count), "r"(1u) : "memory");
     unsigned int polls = 0;
-    while ((int)(ld_acquire_u32(count) - target) < 0) {
+    while (max_polls == 0 || (int)(ld_acquire_u32(count) - target) < 0) {
         if (++polls > max_polls || ((polls & 63u) == 0 && *(volatile int*)err != 0)) {
             atomicExch(err, 1);
             return false;

@@ -158,6 +158,8 @@ struct KrylovWork {
     KrylovScalars* sc = nullptr;     // device scalars (FP64 solve / outer)
     KrylovScalars* sc32 = nullptr;   // device scalars (inner FP32 solve)
     KrylovScalars* host_sc = nullptr;// pinned mirror
+    int32_t* host_wait = nullptr;    // pinned: non-zero after a resident launch one of whose waits gave up
+    int give_up = -1;                // the CTA that gives its waits up (mhfem_check_wait_report; -1: none)
 };
 
 void krylov_init_fp64(const EllMatrix& A, const double* b, double* x, KrylovWork& W,
@@ -243,9 +245,10 @@ bool krylov_resident_fits(int64_t rows, int width, bool fp32);
 // begin; *stop non-zero: it ends at once with KS_ASSEMBLY and x untouched), or
 // goes on with the solve (b null).  W.r, W.rh, W.p, W.v and W.s are work
 // vectors.  The scalars end in W.sc and, when `host` (pinned) is not null, in
-// *host; a launch one of whose waits gave up sets the flag at W.counters +
-// kBarrierError and writes neither.  cudaErrorCooperativeLaunchTooLarge: the
-// device cannot hold the launch at once, and nothing ran.
+// *host.  A launch one of whose waits gave up sets the flag at W.counters +
+// kBarrierError and *W.host_wait (may be null); its scalars and vectors are
+// then void, written or not.  cudaErrorCooperativeLaunchTooLarge: the device
+// cannot hold the launch at once, and nothing ran.
 cudaError_t krylov_resident_fp64(const EllMatrix& A, const double* b, double tol, int max_iter, const int32_t* stop,
                                  double* x, KrylovWork& W, KrylovScalars* host, int iters, cudaStream_t s);
 // The same for the mixed form's inner solve, set up by mixed_inner_init.

@@ -31,8 +31,10 @@
 //    (resident_two.cuh): its barrier takes 0.5 us and the gathers read the
 //    neighbours' shared memory.
 // Every wait on a grid counter is bounded: a CTA that polls kBarrierPolls
-// times records the failure in *bar_err and returns, and the others then fail
-// their waits too.
+// times records the failure in *bar_err and in pinned memory and returns, and
+// the others then fail their next waits.  The first CTA may have passed the
+// last wait and have written a result all the same, so the host looks at the
+// pinned word after every launch, whatever the result says.
 #include <algorithm>
 #include <mutex>
 #include <set>
@@ -60,6 +62,8 @@ struct ResidentArgs {
     double* partials;   // [4 reductions][kSums][CTA]
     unsigned int* bar;  // arrival count, and its value at the last launch's end
     int* bar_err;
+    int* host_wait;     // pinned: set by a CTA whose wait gave up (may be null)
+    int give_up;        // the CTA whose waits give up at once (a check of the report; -1: none)
     int max_its;
 };
 
@@ -133,6 +137,8 @@ struct Group {
     double* partials;
     unsigned int* bar;
     int* err;
+    int* host_wait;
+    unsigned int polls;
     // Arrivals that the counter has seen (in the first warp).  The count runs
     // on from launch to launch: the word behind it holds its value at the last
     // launch's end.
@@ -146,6 +152,14 @@ struct Group {
     __device__ __forceinline__ void end()
     {
         if (!CL && blockIdx.x == 0 && threadIdx.x == 0) bar[1] = target;
+    }
+
+    // One thread of the CTA: arrives and waits for the others.
+    __device__ __forceinline__ void wait()
+    {
+        if (arrive_and_wait(bar, err, target, polls)) return;
+        *bad = 1;
+        if (host_wait) *(volatile int*)host_wait = 1;
     }
 
     // Barrier of the first NV warps.
@@ -202,7 +216,7 @@ struct Group {
                 sum_warps_sync<NV>();
                 if (warp == 0) {
                     target += nc;
-                    if (lane == 0 && !arrive_and_wait(bar, err, target)) *bad = 1;
+                    if (lane == 0) wait();
                 }
                 sum_warps_sync<NV>();
                 const bool ok = *(volatile int*)bad == 0;
@@ -238,7 +252,7 @@ struct Group {
             __syncthreads();
             if (threadIdx.x < 32) {
                 target += gridDim.x;
-                if (threadIdx.x == 0 && !arrive_and_wait(bar, err, target)) *bad = 1;
+                if (threadIdx.x == 0) wait();
             }
             else
                 side((int)(threadIdx.x >> 5) - 1);
@@ -247,6 +261,12 @@ struct Group {
         }
     }
 };
+
+// Polls after which this CTA's waits give up.
+__device__ __forceinline__ unsigned int wait_polls(int give_up)
+{
+    return (int)blockIdx.x == give_up ? 0u : kBarrierPolls;
+}
 
 // Limits that decide a common iteration's end without a square root or a
 // quotient: (tol ||b||)^2 and (kRestartEps ||rh||)^2, each with a margin far
@@ -437,7 +457,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
                 sa[k * rc + m] = __ldg(g.vals + o);
                 scol[k * rc + m] = c;
             }
-    Group<false> G{col, tot, nullptr, &bad, g.partials, g.bar, g.bar_err};
+    Group<false> G{col, tot, nullptr, &bad, g.partials, g.bar, g.bar_err, g.host_wait, wait_polls(g.give_up)};
     G.begin();
     __syncthreads();
 
@@ -894,7 +914,7 @@ cudaError_t iterate_resident(const EllMatrix& A, const R* vals, const R* b, doub
     if (!P.ok || (int64_t)4 * kSums * P.ctas > (int64_t)W.grid * kPartStride) return cudaErrorCooperativeLaunchTooLarge;
     const ResidentArgs<R> a{A.cols, vals, A.width, A.rows, P.rc, x, r, rh, p, v, sv, t, b, tol,
                             max_iter, stop, sc, host, W.partials, W.counters + kBarrierFirst,
-                            reinterpret_cast<int*>(W.counters + kBarrierError), iters};
+                            reinterpret_cast<int*>(W.counters + kBarrierError), W.host_wait, W.give_up, iters};
     if (P.two) return launch_two(A.width, P.cluster, P.ctas, P.threads, P.smem, a, dev, s);
     MHFEM_WIDTH_DISPATCH(A.width, e = (launch_form<R, WW>(P, a, dev, s)));
     return e;
