@@ -1,0 +1,75 @@
+"""The launch shapes of the resident BiCGStab (csrc/resident_plan.h), on the CPU: every plan's
+launch is one that the kernel it names accepts, whatever the system's rows and width."""
+import itertools
+import subprocess
+from pathlib import Path
+
+import pytest
+
+REPO = Path(__file__).resolve().parent.parent
+SMS, SMEM = 152, 227 * 1024
+FIELDS = ("ok", "two", "cluster", "mats", "recomp", "x_in_smem", "ctas", "threads", "rc", "smem", "bound")
+
+
+@pytest.fixture(scope="session")
+def plan(tmp_path_factory):
+    out = tmp_path_factory.mktemp("plan") / "resident_plan_check"
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", "-I", str(REPO / "tnl-mhfem_gb300" / "csrc"),
+                        str(REPO / "tests" / "resident_plan_check.cpp"), "-o", str(out)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+
+    def run(systems):
+        text = "".join(f"{rows} {width} {real} {SMS} {SMEM}\n" for rows, width, real in systems)
+        r = subprocess.run([str(out)], input=text, capture_output=True, text=True)
+        assert r.returncode == 0
+        return [dict(zip(FIELDS, map(int, line.split()))) for line in r.stdout.splitlines()]
+
+    return run
+
+
+def test_every_launch_is_within_its_kernels_bounds(plan):
+    """Block size within the launch bound, whole warps, shared memory within
+    the device's, at most one CTA per SM, every row owned by one CTA."""
+    rows = sorted({r + d for r in [1, 128, 1024, 4096, *range(5000, 1_700_000, 9973), 622_592, 262_144]
+                   for d in (0, 1)})
+    systems = list(itertools.product(rows, [0, 1, 2, 3, 4, 5, 6, 8, 9, 10, 13, 17, 25, 40], [4, 8]))
+    for (r, w, real), P in zip(systems, plan(systems)):
+        if not P["ok"]:
+            continue
+        at = (r, w, real, P)
+        assert P["threads"] <= P["bound"] and P["threads"] % 32 == 0 and P["threads"] >= 128, at
+        assert P["smem"] <= SMEM, at
+        assert 1 <= P["ctas"] <= (16 if P["cluster"] else SMS), at
+        assert P["ctas"] * P["rc"] >= r, at
+        if not P["cluster"]:
+            assert (P["ctas"] - 1) * P["rc"] < r, at
+
+
+@pytest.mark.gpu
+def test_mixed_form_without_off_diagonal_entries():
+    """217,800 triangles that share no face, every face Dirichlet: 653,400 rows of ELL width 0, the
+    widest CTAs of the mixed form's inner solve.  The traces are the boundary values."""
+    import numpy as np
+    from helpers import rel_err, variant
+    from mhfem import _lib as L
+    from mhfem import problems
+    from oracle.oracle import OracleModel
+
+    p = variant(problems.heat2d(N=330, steps=1), form=L.FORM_MIXED)
+    p.coords = p.coords[p.cells.ravel()]
+    p.cells = np.arange(3 * p.C, dtype=p.cells.dtype).reshape(-1, 3)
+    p.tol = 1e-13
+
+    def bc(face_verts, face_cells):
+        F = face_cells.shape[0]
+        return np.zeros(F, np.uint8), np.zeros(F), np.linspace(-0.7, 1.1, F)
+
+    p.bc_fn = bc
+    s = problems.make_solver(p)
+    assert s.F == 653_400
+    assert s.step(0.0, p.dt)["residual"] < 1e-13
+    m = OracleModel.from_problem(p)
+    m.step(0.0, p.dt, 1e-13)
+    zf, zk = s.state()
+    assert rel_err(zf, m.Z_iF) < 1e-10 and rel_err(zk, m.Z_iK) < 1e-10
+    s.close()

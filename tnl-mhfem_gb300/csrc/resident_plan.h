@@ -1,0 +1,113 @@
+#pragma once
+// Launch shapes of the resident BiCGStab (resident.cuh, resident_two.cuh): which
+// form takes a system, with how many CTAs and threads and how much shared
+// memory.  Host code without CUDA, so that the rules are tested on the CPU.
+#include <algorithm>
+#include <cstddef>
+#include <cstdint>
+
+namespace mhfem {
+
+// Launch bounds of the kernels: threads of a CTA at most.
+constexpr int kMaxThreads = 512;   // three reductions, streamed
+constexpr int kPassThreads = 384;  // two reductions; elsewhere the most for a CTA whose rows are few (group_threads)
+constexpr int kSums = 4;           // sums of the widest reduction
+constexpr int kMaxCluster = 16;
+
+// Rows up to which one cluster takes the system: its barrier costs half of the
+// grid's, its 16 SMs have a tenth of the FP64 units.  Measured per iteration,
+// cluster and grid: 6.5 and 8.7 us at 800 rows (width 4), 7.8 and 8.8 at 3,960,
+// 8.6 and 8.6 at 5,376, 10.6 and 8.7 at 7,905; 9.1 and 10.6 at 2,480 (width 9),
+// 12.0 and 10.9 at 5,520.
+constexpr int64_t kClusterRows = 4096;
+// Off-diagonal entries up to which phase B of the FP64 solve forms the
+// neighbours' s itself: a barrier less against one FP64 operation per entry.
+// Measured per iteration, with and without: 14.97 and 15.84 us at 0.30M
+// entries (50,688 rows, width 6), 18.5 and 19.0 at 0.68M, 20.6 and 21.0 at
+// 0.79M (width 4), but 22.3 and 21.4 at 1.22M (width 9), 27.1 and 26.4 at
+// 1.44M.  In FP32 the operation costs nothing: always.
+constexpr int64_t kRecompEntries = 1000000;
+
+// Off-diagonal entries up to which the FP64 solve runs with two reductions
+// per iteration (resident_two.cuh).  Measured per iteration against three:
+// 8.6 and 10.1 us at 50,000 entries (width 4), 11.7 and 12.8 at 304,000 (width
+// 6), 13.7 and 14.5 at 432,000, 15.4 and 15.4 at 537,000, but 17.0 and 16.4 at
+// 683,000, 16.9 and 15.8 at 682,000 (width 10).  In FP32 wherever it fits (12.6
+// and 14.7 at 788,000).
+constexpr int64_t kTwoEntries = 500000;
+
+// Matrix bytes up to which the ELL words are streamed from L2 by one CTA per
+// SM (129 MB of L2 also holds the gathered vectors and x).  Measured per
+// iteration against the five kernels: 48.7 and 57.3 us at 44 MB (width 6),
+// 55.0 and 64.6 at 56 MB, 45.9 and 64.7 at 64 MB (width 10), but 77.0 and
+// 72.9 at 84 MB (width 9), 80.4 and 76.0 at 87 MB (width 10).
+// In FP32 (with half the vectors' bytes) 42.8 and 56.4 us at 73 MB.
+constexpr int64_t kStreamedBytes = (int64_t)72 << 20;
+
+// Threads of a CTA with `rc` rows: as few passes over them as `most` threads
+// allow, of equal size, whole warps, and at least one warp per FP64 unit.  A
+// thread more is a value more in every block sum, a pass more another round of
+// gather latency.  Measured per iteration: 326 rows 12.4 us with 352 threads
+// (one pass), 13.8 with 192, 14.0 with 256; 793 rows 15.8 with 288 (three),
+// 17.2 with 512, 19.1 with 256; 1,115 rows 18.8 with 384, 20.1 with 512; above
+// 4,096 rows the streamed ELL words want 512 threads (46.7 us against 49.3 with
+// 384 at 5,116 rows, 25.2 and 27.2 in FP32).
+inline int group_threads(int rc, int most)
+{
+    if (rc > 4096) return kMaxThreads;
+    const int passes = (rc + most - 1) / most, per = (rc + passes - 1) / passes;
+    return std::max(128, (per + 31) / 32 * 32);
+}
+
+struct ResidentPlan {
+    bool ok = false, cluster = false, mats = false, recomp = false, x_in_smem = false;
+    bool two = false;  // resident_two.cuh
+    int ctas = 0, threads = 0, rc = 0;
+    size_t smem = 0;
+};
+
+inline ResidentPlan plan_resident(int64_t rows, int width, size_t real, int sms, size_t smem_max)
+{
+    ResidentPlan P;
+    if (rows < 1) return P;
+    auto fill = [&](int ctas) {
+        P.ctas = ctas;
+        P.rc = (int)((rows + ctas - 1) / ctas);
+        P.ctas = (int)((rows + P.rc - 1) / P.rc);  // no empty CTA
+        P.threads = std::min(group_threads(P.rc, kPassThreads), P.two ? kPassThreads : kMaxThreads);
+        const size_t vectors = 5 + (P.recomp ? 1 : 0) + (P.x_in_smem ? 1 : 0);
+        P.smem = sizeof(double) * (size_t)kSums * P.threads + real * vectors * P.rc +
+                 (P.two    ? (real * (1 + 4 * (size_t)width) + sizeof(int32_t) * width) * P.rc
+                  : P.mats ? (real + sizeof(int32_t)) * (size_t)width * P.rc
+                           : 0);
+        return P.smem + 4096 <= smem_max;  // 4 KB for the static shared variables
+    };
+    const int64_t want = (rows + 127) / 128;
+    const int ctas = (int)std::min<int64_t>(want, sms);
+    if (real == 4 || rows * width <= kTwoEntries) {
+        // two reductions per iteration, in a cluster or the grid
+        for (bool cluster : {true, false}) {
+            if (cluster && rows > kClusterRows) continue;
+            P = ResidentPlan{};
+            P.two = P.x_in_smem = true;
+            P.cluster = cluster;
+            int c = 1;
+            while (c < kMaxCluster && (int64_t)c * 128 < rows) c *= 2;
+            P.ok = fill(cluster ? c : ctas);
+            if (cluster) P.ctas = c;  // every CTA of the cluster is launched, also those left without rows
+            if (P.ok) return P;
+        }
+    }
+    for (int form = 0; form < 3; ++form) {  // ELL words and x in shared memory, x only, neither
+        if (form > 0 && (int64_t)(real + 4) * width * rows > kStreamedBytes) return ResidentPlan{};
+        P = ResidentPlan{};
+        P.mats = form == 0;
+        P.recomp = P.mats && (real == 4 || rows * width <= kRecompEntries);
+        P.x_in_smem = form < 2;
+        P.ok = fill(ctas);
+        if (P.ok) return P;
+    }
+    return P;
+}
+
+}  // namespace mhfem
