@@ -359,8 +359,8 @@ mhfem_status mhfem_check_grid_barrier(int32_t device, int32_t ctas, int32_t skip
                                       int32_t* ctas_passed, int32_t* ctas_gave_up, int32_t* failure_flag);
 
 /* Check of the failure report of the resident solves: from now on CTA `cta`
- * of their grid launches (negative: none, the default) gives up each of its
- * waits at once, as a CTA does whose wait ran out.  A solve with such a launch
+ * of their grid launches (negative: none, the default) gives up its first
+ * wait, as a CTA does whose wait ran out.  A solve with such a launch
  * returns MHFEM_ERR_CUDA, whichever wait it was, and the next one (with -1)
  * works again.  Launches of fewer CTAs, one-cluster launches (up to 4,096
  * rows) and the five-kernel iteration have no such wait. */

@@ -1,7 +1,7 @@
 """A wait between the CTAs of a resident solve that gives up is reported,
 whichever wait it was and whatever the first CTA wrote.
 
-mhfem_check_wait_report makes one CTA give its waits up at once: it has
+mhfem_check_wait_report makes one CTA give its waits up: it has
 arrived, so the others pass that wait and fail the next one within a few
 polls.  Nothing hangs: every wait is bounded, and a CTA that gave up returns.
 """

@@ -366,7 +366,7 @@ __device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int* p)
 
 // Adds one arrival to a grid counter (release) and waits until it reaches
 // `target` (acquire; the count grows by one per arrival); one thread.  False
-// when the wait gave up (with max_polls 0: always).  The counter's own
+// when the wait gave up.  The counter's own
 // release and acquire order the CTA's writes before the arrival (behind a
 // __syncthreads) and its reads after the wait, with no thread fence: 1.5
 // instead of 1.9 us for a barrier over 152 CTAs.
@@ -375,7 +375,7 @@ __device__ __forceinline__ bool arrive_and_wait(unsigned int* count, int* err, u
 {
     asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(count), "r"(1u) : "memory");
     unsigned int polls = 0;
-    while (max_polls == 0 || (int)(ld_acquire_u32(count) - target) < 0) {
+    while ((int)(ld_acquire_u32(count) - target) < 0) {
         if (++polls > max_polls || ((polls & 63u) == 0 && *(volatile int*)err != 0)) {
             atomicExch(err, 1);
             return false;
