@@ -1,0 +1,57 @@
+"""How a resident BiCGStab solve ends or restarts when a scalar of the iteration vanishes, in every
+form it runs in: systems of equal small blocks of dyadic numbers, as many as a power of two, through
+mhfem_bicgstab_noalloc.  Every sum, quotient and update below is exact in FP64, so each branch is
+taken for certain.
+"""
+import ctypes as ct
+
+import numpy as np
+import pytest
+
+from mhfem import _lib as L
+
+pytestmark = pytest.mark.gpu
+
+# (rows, ELL width): the form that the plan gives them
+FORMS = [
+    (64, 4),        # one CTA
+    (2048, 6),      # a cluster
+    (16384, 4),     # the grid, two reductions
+    (131072, 4),    # three reductions, phase B forms the neighbours' s
+    (131072, 9),    # three reductions, s published
+    (262144, 10),   # the ELL words streamed
+    (262144, 13),
+]
+
+
+def solve_blocks(block, b, rows, width, tol=1e-12, max_iter=100):
+    """A x = b from x = 0, A = rows / len(b) copies of `block` (unit diagonal) on the diagonal."""
+    import torch
+
+    lib = L.load()
+    block = np.asarray(block, np.float64)
+    n = block.shape[0]
+    assert rows % n == 0 and np.all(np.diag(block) == 1) and width >= n - 1
+    r = np.arange(rows)
+    cols = np.tile(r.astype(np.int32), (width, 1))  # padding: the own row, value 0
+    vals = np.zeros((width, rows))
+    for i in range(n):
+        for k, j in enumerate(j for j in range(n) if j != i):
+            cols[k, i::n] = r[i::n] - i + j
+            vals[k, i::n] = block[i, j]
+    dev = [torch.from_numpy(a).cuda() for a in (cols, vals, np.tile(np.asarray(b, np.float64), rows // n))]
+    x = torch.zeros(rows, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    it, res = ct.c_int32(), ct.c_double()
+    st = lib.mhfem_bicgstab_noalloc(dev[0].data_ptr(), dev[1].data_ptr(), width, rows, dev[2].data_ptr(),
+                                    x.data_ptr(), tol, max_iter, 60.0, ct.byref(it), ct.byref(res), None)
+    return st, it.value, res.value, x.cpu().numpy().reshape(-1, n)
+
+
+@pytest.mark.parametrize("rows,width", FORMS)
+def test_residual_that_vanishes(rows, width):
+    """One unknown of a pair depends on the other: alpha = 1, s = (-a, 0) is not zero, omega = 1 and
+    r = 0 after the first iteration, with (rh, r) = 0 and nothing left to restart from."""
+    st, it, res, x = solve_blocks([[1.0, -0.5], [0.0, 1.0]], [0.0, 1.0], rows, width)
+    assert st == L.OK and it == 1 and res == 0
+    assert np.array_equal(x, np.tile([0.5, 1.0], (rows // 2, 1)))

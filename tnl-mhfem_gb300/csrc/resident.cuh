@@ -306,17 +306,25 @@ __device__ __forceinline__ void end_of_iteration(KrylovScalars* S, EndLimits* li
         S->rho = rho;
 }
 
-// The same after an iteration that did not sum over r: rho' from phase B's
-// sums, the restart test against the last known ||r||, no convergence test.
-__device__ __forceinline__ void end_unchecked(KrylovScalars* S, const EndLimits* lim, double rho)
+// Whether an iteration of the streamed forms can go without sums over r: from
+// phase B's sums, nothing ends it and it does not restart, by
+// end_of_iteration's conditions with the last known ||r||.  Otherwise it sums,
+// so that every end and restart is decided on the residual itself (r may have
+// vanished, and with it rho').  For a thread beside scalars_omega_beta's: it
+// forms omega and rho' again rather than wait for them.
+__device__ __forceinline__ bool plain_iteration(const KrylovScalars* S, const EndLimits* lim, const double* tot)
 {
+    const double omega = tot[0] * recip_newton(tot[1]), rho = fma(-omega, tot[3], tot[2]);
     const double rho2 = rho * rho, bound2 = lim->restart2 * S->rr;
+    return finite_bits(rho2) && greater_bits(bound2, kTiny) && greater_bits(rho2, bound2) && !zero_bits(omega) &&
+           !zero_bits(S->rho);
+}
+
+// The end of such an iteration.
+__device__ __forceinline__ void end_unchecked(KrylovScalars* S, double rho)
+{
     S->it += 1;
-    S->restart = !(finite_bits(rho2) && greater_bits(bound2, kTiny) && greater_bits(rho2, bound2)) &&
-                 fabs(rho) <= kRestartEps * sqrt(S->rr) * S->rhnorm;
-    if (!finite_bits(rho)) { S->status = KS_NOTFINITE; S->done = 1; }
-    else if (zero_bits(S->omega) || zero_bits(S->rho)) { S->status = KS_BREAKDOWN; S->done = 1; }
-    if (S->done) S->res = sqrt(S->rr) / S->bnorm;
+    S->restart = 0;
     S->rho = rho;
 }
 
@@ -414,6 +422,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
     __shared__ KrylovScalars S;
     __shared__ double tot[kSums];
     __shared__ double s_inv_rv, s_rho_next;
+    __shared__ int s_plain;
     __shared__ int bad;
     const int T = blockDim.x, rc = g.rc, W = WW > 0 ? WW : g.W;
     const int64_t base = (int64_t)blockIdx.x * rc, rows = g.rows;
@@ -635,6 +644,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
             }
             if (!G.reduce(acc, 1)) return;
             if (threadIdx.x == 0 || threadIdx.x == 32) scalars_omega_beta(&S, tot, s_inv_rv, &s_rho_next);
+            else if (!MATS && threadIdx.x == 64) s_plain = plain_iteration(&S, &limits, tot);
             __syncthreads();
             if (S.done) break;
         }
@@ -649,7 +659,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
         // C. r, p (and x, while the sums go round), (r, r), (rh, r) -> convergence, restart
         {
             const R omega = (R)S.omega, beta = (R)S.beta;
-            const bool check = MATS || (S.it + 1) % kStreamedCheckEvery == 0 || k + 1 == g.max_its ||
+            const bool check = MATS || !s_plain || (S.it + 1) % kStreamedCheckEvery == 0 || k + 1 == g.max_its ||
                                S.it + 1 >= S.max_iter;
             R acc[2] = {0, 0};
             R* const rnew = RECOMP ? sr : st;
@@ -673,7 +683,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
             }
             else {
                 if (!G.barrier([&](int w) { if (side_x) add_to_x(omega, ss, w, 1); })) return;
-                if (threadIdx.x == 0) end_unchecked(&S, &limits, s_rho_next);
+                if (threadIdx.x == 0) end_unchecked(&S, s_rho_next);
             }
             if constexpr (!RECOMP) {  // r is where t was; the next s takes its place, the next t that of this s
                 st = ss;
