@@ -113,9 +113,11 @@ typedef struct {
     double  inner_tol;        /* mixed form: relative tolerance of each FP32 sweep */
     int32_t max_sweeps;       /* mixed form: cap on refinement sweeps */
     int32_t check_every;      /* Krylov iterations between host convergence checks (systems
-                                 too large for the SMs; an FP64 BiCGStab solve of up to
-                                 about 800,000 rows runs resident on them and tests every
-                                 iteration, above about 340,000 rows every fourth) */
+                                 too large for the SMs; an FP64 BiCGStab solve of up to about
+                                 800,000 rows with at most 72 MB of matrix entries runs resident
+                                 on them and tests its convergence in every iteration up to
+                                 2^18 rows, and above while the entries fit the SMs' shared
+                                 memory (340,000 rows of 4), else in every fourth) */
     double  timeout_s;        /* host wall-clock limit of one solve (<= 0: none) */
     int32_t inner_adaptive;   /* mixed form: relax the last sweeps' inner tolerance to what the outer
                                  tolerance still needs (never tighter than inner_tol) */

@@ -10,9 +10,10 @@
 //
 // The Krylov work vectors, the per-CTA partial sums and the device scalars
 // live in one file-scope static device array of fixed size (about 13 MB).
-// Every system it takes fits the resident solve (k_resident.cu: one launch
-// per chunk of 256 iterations, the convergence test in every iteration),
-// which mhfem_solve runs for the same sizes.
+// Every system it takes, whatever its width, runs the resident solve
+// (k_resident.cu: one launch per chunk of 256 iterations, the convergence test
+// in every iteration up to kEveryTestRows rows), which mhfem_solve runs for the
+// same systems.
 // Under CUDA's lazy module loading the array is committed on a device at the
 // first call there (the cudaGetSymbolAddress below loads the module), not when
 // the library is loaded, and it stays until the process exits; systems with
@@ -22,9 +23,11 @@
 
 #include "handle.h"
 #include "mhfem_internal.h"
+#include "resident_plan.h"
 
 namespace {
 
+static_assert(MHFEM_NOALLOC_MAX_ROWS <= mhfem::kEveryTestRows, "every system runs resident and tests every iteration");
 constexpr int64_t kMaxRows = MHFEM_NOALLOC_MAX_ROWS;   // even: the vectors below are spaced by an even count
 constexpr int64_t kMaxGrid = 4096;                     // per-CTA partials (>= any Krylov grid here)
 constexpr int64_t kVecDoubles = 6 * kMaxRows;          // r, rh, p, v, s, t

@@ -66,6 +66,7 @@ struct ResidentArgs {
     int* host_wait;     // pinned: set by a CTA whose wait gave up (may be null)
     int give_up;        // the CTA whose waits give up (a check of the report; -1: none)
     int max_its;
+    int check_mask;     // streamed forms: iterations between the sums over r, less one (1, 2, 4, ... less one)
 };
 
 namespace {
@@ -406,11 +407,6 @@ __device__ __forceinline__ void scalars_half_step(KrylovScalars* S)
     S->done = 1;
 }
 
-// Iterations between the convergence tests of the streamed forms.  There the
-// FP64 pipe bounds the vector phases, and the two sums over r are two of 26
-// operations per row; a solve takes hundreds of iterations.
-constexpr int kStreamedCheckEvery = 4;
-
 // WW: compile-time ELL width (0: run-time).  MATS: the CTA's ELL words are
 // copied to shared memory once.  RECOMP: phase B forms s at each gathered neighbour from its
 // r and v (W more FP64 operations per row) instead of publishing s behind a
@@ -659,7 +655,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
         // C. r, p (and x, while the sums go round), (r, r), (rh, r) -> convergence, restart
         {
             const R omega = (R)S.omega, beta = (R)S.beta;
-            const bool check = MATS || !s_plain || (S.it + 1) % kStreamedCheckEvery == 0 || k + 1 == g.max_its ||
+            const bool check = MATS || !s_plain || ((S.it + 1) & g.check_mask) == 0 || k + 1 == g.max_its ||
                                S.it + 1 >= S.max_iter;
             R acc[2] = {0, 0};
             R* const rnew = RECOMP ? sr : st;
@@ -821,7 +817,8 @@ cudaError_t iterate_resident(const EllMatrix& A, const R* vals, const R* b, doub
     if (!P.ok || (int64_t)4 * kSums * P.ctas > (int64_t)W.grid * kPartStride) return cudaErrorCooperativeLaunchTooLarge;
     const ResidentArgs<R> a{A.cols, vals, A.width, A.rows, P.rc, x, r, rh, p, v, sv, t, b, tol,
                             max_iter, stop, sc, host, W.partials, W.counters + kBarrierFirst,
-                            reinterpret_cast<int*>(W.counters + kBarrierError), W.host_wait, W.give_up, iters};
+                            reinterpret_cast<int*>(W.counters + kBarrierError), W.host_wait, W.give_up, iters,
+                            P.check_every - 1};
     if (P.two) return launch_two(A.width, P.cluster, P.ctas, P.threads, P.smem, a, dev, s);
     MHFEM_WIDTH_DISPATCH(A.width, e = (launch_form<R, WW>(P, a, dev, s)));
     return e;

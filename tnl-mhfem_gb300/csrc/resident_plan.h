@@ -59,9 +59,25 @@ inline int group_threads(int rc, int most)
     return std::max(128, (per + 31) / 32 * 32);
 }
 
+// Rows up to which every FP64 system runs resident, whatever its width, and
+// tests its convergence in every iteration: MHFEM_NOALLOC_MAX_ROWS, the size up
+// to which mhfem_bicgstab_noalloc promises both.  The test costs the streamed
+// forms 1.0 to 1.5 us per iteration there (227,556 rows of width 10 24.9 ->
+// 25.9 us, 262,144 of width 13 29.1 -> 30.6).  The ELL words of the widest
+// systems exceed kStreamedBytes: 45.1 us per iteration against the five
+// kernels' 123.5 at 262,144 rows of width 25, 98.3 against 175.7 at width 40.
+constexpr int64_t kEveryTestRows = (int64_t)1 << 18;
+
+// Iterations between the convergence tests of the streamed forms above
+// kEveryTestRows (a power of two).  There the FP64 pipe bounds the vector
+// phases, and the two sums over r are two of 26 operations per row; a solve
+// takes hundreds of iterations.
+constexpr int kStreamedCheckEvery = 4;
+
 struct ResidentPlan {
     bool ok = false, cluster = false, mats = false, recomp = false, x_in_smem = false;
     bool two = false;  // resident_two.cuh
+    int check_every = 1;
     int ctas = 0, threads = 0, rc = 0;
     size_t smem = 0;
 };
@@ -98,9 +114,11 @@ inline ResidentPlan plan_resident(int64_t rows, int width, size_t real, int sms,
             if (P.ok) return P;
         }
     }
+    const bool every = real == 8 && rows <= kEveryTestRows;
     for (int form = 0; form < 3; ++form) {  // ELL words and x in shared memory, x only, neither
-        if (form > 0 && (int64_t)(real + 4) * width * rows > kStreamedBytes) return ResidentPlan{};
+        if (form > 0 && !every && (int64_t)(real + 4) * width * rows > kStreamedBytes) return ResidentPlan{};
         P = ResidentPlan{};
+        P.check_every = form == 0 || every ? 1 : kStreamedCheckEvery;
         P.mats = form == 0;
         P.recomp = P.mats && (real == 4 || rows * width <= kRecompEntries);
         P.x_in_smem = form < 2;
