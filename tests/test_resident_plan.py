@@ -8,7 +8,7 @@ import pytest
 
 REPO = Path(__file__).resolve().parent.parent
 SMS, SMEM = 152, 227 * 1024
-FIELDS = ("ok", "two", "cluster", "mats", "recomp", "x_in_smem", "ctas", "threads", "rc", "smem", "bound")
+FIELDS = ("ok", "two", "cluster", "mats", "recomp", "x_in_smem", "ctas", "threads", "rc", "smem", "bound", "gmres")
 
 
 @pytest.fixture(scope="session")
@@ -43,6 +43,15 @@ def test_every_launch_is_within_its_kernels_bounds(plan):
         assert P["ctas"] * P["rc"] >= r, at
         if not P["cluster"]:
             assert (P["ctas"] - 1) * P["rc"] < r, at
+
+
+def test_gmres_route_follows_rows_and_width(plan):
+    """On the faster side at the sizes where both routes were measured, and resident up to 2^18 rows
+    whatever the width."""
+    resident = [(262_144, 4), (262_144, 40), (766_085, 4), (720_954, 6), (694_960, 9), (595_428, 13), (287_712, 21)]
+    kernels = [(786_433, 4), (779_040, 9), (726_516, 13), (455_112, 21), (677_376, 21)]
+    plans = plan([(r, w, 8) for r, w in resident + kernels])
+    assert [P["gmres"] for P in plans] == [1] * len(resident) + [0] * len(kernels)
 
 
 @pytest.mark.gpu

@@ -12,6 +12,7 @@
 
 #include "gmres_restart.h"
 #include "mhfem_internal.h"
+#include "resident_plan.h"
 #include "topology.h"
 
 using namespace mhfem;
@@ -718,7 +719,7 @@ mhfem_status run_gmres(mhfem_t h, double tol, int max_iter, const int32_t* stop,
     h->launches += 1;
     CK(cudaGetLastError());
     const bool reorth = h->opts.gmres_variant == MHFEM_GMRES_CGSR;
-    if (rows <= krylov_small_rows()) {
+    if (gmres_resident_fits(rows, h->A.width)) {
         // the system fits: chunks of iterations, restarts included, in one
         // launch each (k_gmres_resident.cu), one host round trip per chunk;
         // the device applies the restart rule

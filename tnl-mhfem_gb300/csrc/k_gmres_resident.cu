@@ -1,5 +1,5 @@
-// Restarted GMRES resident on the SMs (sm_103a, FP64), for systems of at most
-// krylov_small_rows() rows: one launch runs up to `max_its` Arnoldi
+// Restarted GMRES resident on the SMs (sm_103a, FP64), for the systems of
+// gmres_resident_fits: one launch runs up to `max_its` Arnoldi
 // iterations, restarts included.  CTAs, rows, clusters, reductions and bounded
 // waits are those of the resident BiCGStab (resident.cuh); the algorithm, the
 // unnormalized basis (v_i = inv_i u_i) and the solve state are k_gmres.cu's.

@@ -1237,16 +1237,7 @@ void krylov_fp64_kernel_once(const EllMatrix& A, KrylovWork& W, int which, cudaS
 }
 
 
-// ---- small systems: host side ----------------------------------------------------
-
-// Rows up to which GMRES runs resident (k_gmres_resident.cu).  Measured per
-// iteration (restart length up to 30) against the two kernels of k_gmres.cu:
-// 36.7 and 81.6 us at 270,600 rows, 55.8 and 91.6 at 437,778, 102.5 and 115.2
-// at 667,128, 103.1 and 110.3 at 751,000: with the basis in memory both come
-// to be bound by its traffic.
-constexpr int64_t kSmallSystemRows = (int64_t)3 << 18;
-
-int64_t krylov_small_rows() { return kSmallSystemRows; }
+// ---- check of the bounded grid wait: host side -----------------------------------
 
 cudaError_t grid_barrier_check(int ctas, int skip, unsigned int max_polls, int* passed, int* gave_up, int* flag)
 {

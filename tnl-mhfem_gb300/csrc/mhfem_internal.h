@@ -221,15 +221,13 @@ void gmres_init(const EllMatrix& A, const double* b, const double* x, GmresWork&
 void gmres_iterate(const EllMatrix& A, GmresWork& G, KrylovWork& W, int iters, bool reorth, cudaStream_t s);
 // end of a cycle: solve the triangular system and update x
 void gmres_update(double* x, GmresWork& G, int64_t rows, cudaStream_t s);
-// Small systems (at most krylov_small_rows() rows): up to `iters` Arnoldi
+// Systems of gmres_resident_fits (resident_plan.h): up to `iters` Arnoldi
 // iterations, restarts included, in one launch (k_gmres_resident.cu) on a
 // solve set up by gmres_init; G.host gets the control words, as *host of
 // krylov_resident_fp64 the scalars.
 cudaError_t gmres_resident(const EllMatrix& A, const double* b, double* x, GmresWork& G, KrylovWork& W, bool reorth,
                            int iters, cudaStream_t s);
 void krylov_iterate_fp64(const EllMatrix& A, double* x, KrylovWork& W, int iters, cudaStream_t s);
-// Rows up to which GMRES runs resident.
-int64_t krylov_small_rows();
 // Words of KrylovWork::counters: [0] the reductions' ticket, [3] the flag of a
 // resident solve's wait that gave up, then (on a 128-byte line of its own) the
 // resident solves' arrival count and its value at the end of the last launch.

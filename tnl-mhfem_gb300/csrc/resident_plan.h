@@ -1,7 +1,7 @@
 #pragma once
 // Launch shapes of the resident BiCGStab (resident.cuh, resident_two.cuh): which
 // form takes a system, with how many CTAs and threads and how much shared
-// memory.  Host code without CUDA, so that the rules are tested on the CPU.
+// memory; and which systems the resident GMRES takes.  Host code without CUDA, so that the rules are tested on the CPU.
 #include <algorithm>
 #include <cstddef>
 #include <cstdint>
@@ -126,6 +126,29 @@ inline ResidentPlan plan_resident(int64_t rows, int width, size_t real, int sms,
         if (P.ok) return P;
     }
     return P;
+}
+
+// Whether restarted GMRES runs resident (k_gmres_resident.cu).  Above about
+// 90,000 rows the basis and the ELL words are read from memory, by one CTA per
+// SM against up to eight of k_gmres.cu's kernels, so the route follows the bytes
+// of the matrix and of a part of the basis.  Measured per iteration, resident
+// and two kernels, with restart length 5 and 30 (in brackets rows x (12 width +
+// 100) in millions):
+//   288,920 rows, width  4  (43): 20.3 and 45.3 us, 39.6 and 81.9
+//   287,712 rows, width 21 (101): 49.1 and 76.0, 74.7 and 107.6
+//   766,085 rows, width  4 (113): 48.4 and 64.1, 131.4 and 134.7
+//   720,954 rows, width  6 (124): 49.9 and 67.4, 128.8 and 135.2
+//   694,960 rows, width  9 (145): 62.5 and 73.9, 133.3 and 140.0
+//   595,428 rows, width 13 (152): 71.3 and 74.5, 122.4 and 129.4
+//   but 455,112, width 21 (160): 102.2 and 88.4, 130.0 and 130.2
+//   779,040 rows, width  9 (162): 77.4 and 76.0, 153.9 and 146.3
+//   726,516 rows, width 13 (186): 87.6 and 84.7, 149.3 and 145.0
+//   677,376 rows, width 21 (238): 150.4 and 96.6, 198.7 and 157.3
+// Up to 2^18 rows always: only a width above 40 would exceed the line there.
+inline bool gmres_resident_fits(int64_t rows, int width)
+{
+    if (rows <= ((int64_t)1 << 18)) return true;
+    return rows <= ((int64_t)3 << 18) && rows * (12 * (int64_t)width + 100) <= 155000000;
 }
 
 }  // namespace mhfem
