@@ -324,8 +324,12 @@ __global__ void __launch_bounds__(NT, TRAIN ? 2 : 3) k_mpnn_layer(const MpnnView
 // rows and writes four gradients per instruction); the FP64 loss arithmetic of
 // the warp's 32 faces then runs once, a face to a lane.  A row per thread
 // touched 32 rows per instruction and took 104 us at 777,600 faces (43% of
-// HBM for the 392 bytes a face).
-__global__ void __launch_bounds__(256) k_mpnn_decode(const MpnnView V, const double* target, double inv_nt)
+// HBM for the 392 bytes a face).  The weight gradient's sums are FP32 over the
+// warp's 32 faces, in runs of four and three levels of pairs (the last two
+// over the row groups, halving the values that a lane holds, so that a lane
+// adds two and not eight FP64 values per 32 faces), and FP64 from there on:
+// their error does not grow with the mesh.
+__global__ void __launch_bounds__(256, 2) k_mpnn_decode(const MpnnView V, const double* target, double inv_nt)
 {
     __shared__ double red[256 / 32][H + 2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -335,7 +339,8 @@ __global__ void __launch_bounds__(256) k_mpnn_decode(const MpnnView V, const dou
     for (int q = 0; q < 8; ++q) wd[q] = V.wd[8 * j + q];
     const float bd = V.bd[0];
     double acc_l = 0, acc_db = 0;
-    float acc_w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    const bool hi4 = (g & 1) != 0, hi2 = (g & 2) != 0;
+    double acc_w[2] = {0, 0};  // columns 8j + 4 (g & 1) + (g & 2) + {0, 1}
     const __nv_bfloat16* h4 = V.h[kMpnnLayers + 1];
     auto unpack8 = [](const uint4& v, float (&f)[8]) {
         const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
@@ -371,6 +376,7 @@ __global__ void __launch_bounds__(256) k_mpnn_decode(const MpnnView V, const dou
         acc_l = fma(diff, diff, acc_l);
         const float dmine = (float)(2.0 * diff * inv_nt);
         acc_db += dmine;
+        float w[2][8] = {};
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const float dout = __shfl_sync(0xffffffffu, dmine, (lane & 24) | i);
@@ -378,7 +384,7 @@ __global__ void __launch_bounds__(256) k_mpnn_decode(const MpnnView V, const dou
             unpack8(v[i], hv);
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
-                acc_w[q] = fmaf(dout, hv[q], acc_w[q]);
+                w[i / 4][q] = fmaf(dout, hv[q], w[i / 4][q]);
                 d[q] = dout * wd[q];
             }
             const int64_t row = base + 4 * i + g;
@@ -388,15 +394,22 @@ __global__ void __launch_bounds__(256) k_mpnn_decode(const MpnnView V, const dou
                 dh[1] = make_float4(d[4], d[5], d[6], d[7]);
             }
         }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) w[0][q] += w[1][q];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float send = hi4 ? w[0][q] : w[0][q + 4], keep = hi4 ? w[0][q + 4] : w[0][q];
+            w[1][q] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const float send = hi2 ? w[1][q] : w[1][q + 2], keep = hi2 ? w[1][q + 2] : w[1][q];
+            acc_w[q] += f32_to_f64(keep + __shfl_xor_sync(0xffffffffu, send, 16));
+        }
     }
     // block reduction of (dwd[64], dbd, loss) into partials[block][66]
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        float v = acc_w[q];
-        v += __shfl_xor_sync(0xffffffffu, v, 8);
-        v += __shfl_xor_sync(0xffffffffu, v, 16);
-        if (g == 0) red[warp][8 * j + q] = v;
-    }
+    for (int q = 0; q < 2; ++q) red[warp][8 * j + (hi4 ? 4 : 0) + (hi2 ? 2 : 0) + q] = acc_w[q];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         acc_db += __shfl_down_sync(0xffffffffu, acc_db, o);
