@@ -55,3 +55,16 @@ def test_residual_that_vanishes(rows, width):
     st, it, res, x = solve_blocks([[1.0, -0.5], [0.0, 1.0]], [0.0, 1.0], rows, width)
     assert st == L.OK and it == 1 and res == 0
     assert np.array_equal(x, np.tile([0.5, 1.0], (rows // 2, 1)))
+
+
+@pytest.mark.parametrize("rows,width", FORMS)
+def test_right_hand_side_near_the_smallest_numbers(rows, width):
+    """The same system with (rh, v) = 2^-1026: its reciprocal is beyond the largest number, the
+    quotient rho / (rh, v) = 1 is not."""
+    n = rows // 2
+    w = 2.0 ** ((-1026 - int(np.log2(n))) // 2)
+    scale = n * w * w
+    assert scale in (2.0**-1026, 2.0**-1027)
+    st, it, res, x = solve_blocks([[1.0, -0.5], [0.0, 1.0]], [0.0, w], rows, width)
+    assert st == L.OK and it == 1 and res == 0
+    assert np.array_equal(x, np.tile([0.5 * w, w], (n, 1)))

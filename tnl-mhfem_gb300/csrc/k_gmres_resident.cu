@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kGmresThreads, 1) k_gmres_resident(const Gmres
         if (blockIdx.x == 0 && threadIdx.x == 0) *g.host = S.ctl;
         return;
     }
-    if (threadIdx.x == 0) inv_bnorm = 1.0 / S.ctl.bnorm;
+    if (threadIdx.x == 0) inv_bnorm = recip_newton(S.ctl.bnorm);
 
     double* col = smem;
     double* su = col + kSums * T;  // [vectors][rc]
@@ -310,11 +310,16 @@ __global__ void __launch_bounds__(kGmresThreads, 1) k_gmres_resident(const Gmres
                 const double a = S.H[j][j], invj = S.inv[j], sum = tot[0];
                 const double den2 = fma(a, a, (invj * invj) * sum);
                 const double r = sqrt(lane == 0 ? sum : den2), ri = r > 0 ? recip_newton(r) : 0.0;
-                const double nrm = __shfl_sync(0xffffffffu, r, 0), inv = __shfl_sync(0xffffffffu, ri, 0);
+                const double nrm = __shfl_sync(0xffffffffu, r, 0), nrmi = __shfl_sync(0xffffffffu, ri, 0);
                 const double den = __shfl_sync(0xffffffffu, r, 1), deni = __shfl_sync(0xffffffffu, ri, 1);
                 const double hn = invj * nrm;  // h_{j+1,j}
-                const double cs = den > 0 ? a * deni : 1.0, sn = den > 0 ? hn * deni : 0.0;
-                const double gj = S.g[j], gn = -sn * gj, res = fabs(gn) * inv_bnorm;
+                // the rotation's cosine and sine and 1 / ||u|| in one pass, a quotient to a lane
+                const double top = lane == 0 ? a : lane == 1 ? hn : 1.0, bot = lane < 2 ? den : nrm;
+                const double val = bot > 0 ? quotient(top, bot, lane < 2 ? deni : nrmi) : lane == 0 ? 1.0 : 0.0;
+                const double cs = __shfl_sync(0xffffffffu, val, 0), sn = __shfl_sync(0xffffffffu, val, 1);
+                const double inv = __shfl_sync(0xffffffffu, val, 2);
+                // the estimate that ends the cycle; the residual that is reported is formed at the restart
+                const double gj = S.g[j], gn = -sn * gj, res = quotient_product(fabs(gn), S.ctl.bnorm, inv_bnorm);
                 __syncwarp();
                 if (lane == 0) {
                     S.cs[j] = cs;
@@ -341,7 +346,7 @@ __global__ void __launch_bounds__(kGmresThreads, 1) k_gmres_resident(const Gmres
             double gi = lane < k ? S.g[lane] : 0.0, y = 0;
             const double ri = lane < k ? recip_newton(S.H[lane][lane]) : 0.0;
             for (int i = k - 1; i >= 0; --i) {
-                const double yi = __shfl_sync(0xffffffffu, gi * ri, i);
+                const double yi = __shfl_sync(0xffffffffu, lane < k ? quotient(gi, S.H[lane][lane], ri) : 0.0, i);
                 if (lane == i) y = yi;
                 if (lane < i) gi = fma(-S.H[lane][i], yi, gi);
             }

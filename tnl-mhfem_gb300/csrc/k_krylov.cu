@@ -365,9 +365,8 @@ __device__ __forceinline__ void stream_groups(int64_t nv, const T* const (&in)[K
 }
 
 // The scalars between the phases are one thread's work in a kernel's tail, 64
-// cycles per FP64 operation: reciprocals of three operations (recip_newton)
-// instead of divisions of nine, tests on bit patterns, no square root outside
-// check iterations.
+// cycles per FP64 operation: quotients of six operations (fp_recip.h), tests on
+// bit patterns, no square root outside check iterations.
 
 // alpha = rho / (rh, v)
 __device__ __forceinline__ void scalars_alpha(KrylovScalars* sc, const double (&s)[1])
@@ -375,7 +374,7 @@ __device__ __forceinline__ void scalars_alpha(KrylovScalars* sc, const double (&
     sc->rv = s[0];
     if (!finite_bits(s[0])) { sc->status = KS_NOTFINITE; sc->done = 1; }
     else if (zero_bits(s[0])) { sc->status = KS_BREAKDOWN; sc->done = 1; }
-    else sc->alpha = sc->rho * recip_newton(s[0]);
+    else sc->alpha = quotient(sc->rho, s[0]);
 }
 
 // s = r - alpha v
@@ -516,7 +515,7 @@ __device__ __forceinline__ void scalars_omega(KrylovScalars* sc, const double (&
             sc->half = 1;
         }
     }
-    else sc->omega = sum[0] * recip_newton(sum[1]);
+    else sc->omega = quotient(sum[0], sum[1]);
 }
 
 // half step: x += alpha p
@@ -613,7 +612,7 @@ __device__ __forceinline__ void scalars_beta(KrylovScalars* sc, const double (&s
     }
     else {
         sc->restart = 0;
-        sc->beta = (sum[0] * recip_newton(rho)) * (sc->alpha * recip_newton(omega));
+        sc->beta = quotient(sum[0], rho) * quotient(sc->alpha, omega);
         sc->rho = sum[0];
     }
 }

@@ -25,8 +25,8 @@
 //  - a reduction's sums go to different warps (one per FP64 unit of the SM),
 //    with one arrival and one polling thread per CTA and no thread fence beyond
 //    the counter's own release and acquire;
-//  - the scalars take one reciprocal of three dependent operations per
-//    reduction, square roots only near the decisions they belong to;
+//  - the scalars take one quotient of six dependent operations per reduction
+//    (fp_recip.h), square roots only near the decisions they belong to;
 //  - the systems of a few thousand rows run in one thread-block cluster
 //    (resident_two.cuh): its barrier takes 0.5 us and the gathers read the
 //    neighbours' shared memory.
@@ -315,7 +315,7 @@ __device__ __forceinline__ void end_of_iteration(KrylovScalars* S, EndLimits* li
 // forms omega and rho' again rather than wait for them.
 __device__ __forceinline__ bool plain_iteration(const KrylovScalars* S, const EndLimits* lim, const double* tot)
 {
-    const double omega = tot[0] * recip_newton(tot[1]), rho = fma(-omega, tot[3], tot[2]);
+    const double omega = quotient(tot[0], tot[1]), rho = fma(-omega, tot[3], tot[2]);
     const double rho2 = rho * rho, bound2 = lim->restart2 * S->rr;
     return finite_bits(rho2) && greater_bits(bound2, kTiny) && greater_bits(rho2, bound2) && !zero_bits(omega) &&
            !zero_bits(S->rho);
@@ -378,8 +378,9 @@ __device__ __forceinline__ void scalars_omega_beta(KrylovScalars* S, const doubl
 {
     const double ts = tot[0], tt = tot[1];
     const double num = threadIdx.x == 0 ? ts : tt, den = threadIdx.x == 0 ? tt : ts;
-    const double q = num * recip_newton(den);
+    const double r = recip_newton(den);
     if (threadIdx.x == 0) {
+        const double q = quotient(num, den, r);
         S->ts = ts;
         S->tt = tt;
         S->omega = q;
@@ -394,8 +395,10 @@ __device__ __forceinline__ void scalars_omega_beta(KrylovScalars* S, const doubl
         else if (zero_bits(tt)) S->half = 1;
     }
     else
-        // beta = (rho' / rho) (alpha / omega) with alpha = rho / (rh, v)
-        S->beta = fma(tot[2], q, -tot[3]) * inv_rv;
+        // beta = (rho' / rho) (alpha / omega) with alpha = rho / (rh, v).  (rh, s) is
+        // zero but for rounding, by the choice of alpha: its factor 1 / omega needs
+        // no correction.
+        S->beta = quotient(fma(tot[2], quotient_product(num, den, r), -tot[3]), S->rv, inv_rv);
 }
 
 __device__ __forceinline__ void scalars_half_step(KrylovScalars* S)
@@ -573,7 +576,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
             if (threadIdx.x == 0) {
                 const double rv = tot[0], inv = recip_newton(rv);
                 S.rv = rv;
-                S.alpha = S.rho * inv;
+                S.alpha = quotient(S.rho, rv, inv);
                 s_inv_rv = inv;
                 if (!finite_bits(rv) || zero_bits(rv)) {
                     S.status = finite_bits(rv) ? KS_BREAKDOWN : KS_NOTFINITE;

@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kPassThreads, 1) k_bicgstab_two(const Resident
             else if (threadIdx.x == 32) {
                 const double rv = tot[0], inv = recip_newton(rv);
                 S.rv = rv;
-                S.alpha = rho * inv;
+                S.alpha = quotient(rho, rv, inv);
                 s_inv_rv = inv;
                 s_rv_status = !finite_bits(rv) ? KS_NOTFINITE : zero_bits(rv) ? KS_BREAKDOWN : KS_RUNNING;
             }
