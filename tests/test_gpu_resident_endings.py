@@ -68,3 +68,19 @@ def test_right_hand_side_near_the_smallest_numbers(rows, width):
     st, it, res, x = solve_blocks([[1.0, -0.5], [0.0, 1.0]], [0.0, w], rows, width)
     assert st == L.OK and it == 1 and res == 0
     assert np.array_equal(x, np.tile([0.5 * w, w], (n, 1)))
+
+
+@pytest.mark.parametrize("rows,width", FORMS)
+def test_half_step_that_does_not_solve(rows, width):
+    """A singular system: alpha = 1/2, s = (-6, 3) and A s = 0.  There is no omega, and ||s|| is three
+    quarters of ||b||: a breakdown, not a solution."""
+    st, it, res, x = solve_blocks([[1.0, 2.0], [0.5, 1.0]], [4.0, 8.0], rows, width)
+    assert st == L.ERR_BREAKDOWN
+
+
+@pytest.mark.parametrize("rows,width", FORMS)
+def test_half_step_that_solves(rows, width):
+    """The identity: alpha = 1 and s = 0, so the first half step solves the system."""
+    st, it, res, x = solve_blocks([[1.0, 0.0], [0.0, 1.0]], [1.0, -1.0], rows, width)
+    assert st == L.OK and it == 1 and res == 0
+    assert np.array_equal(x, np.tile([1.0, -1.0], (rows // 2, 1)))

@@ -391,7 +391,7 @@ __device__ __forceinline__ void scalars_omega_beta(KrylovScalars* S, const doubl
             S->done = 1;
             S->res = sqrt(S->rr) / S->bnorm;
         }
-        // A s = 0 with a nonsingular matrix: s = 0, and x + alpha p solves the system
+        // no omega: the solve ends with the half step (scalars_half_step)
         else if (zero_bits(tt)) S->half = 1;
     }
     else
@@ -401,13 +401,23 @@ __device__ __forceinline__ void scalars_omega_beta(KrylovScalars* S, const doubl
         S->beta = quotient(fma(tot[2], quotient_product(num, den, r), -tot[3]), S->rv, inv_rv);
 }
 
-__device__ __forceinline__ void scalars_half_step(KrylovScalars* S)
+// A s = 0, with ss = (s, s): with a nonsingular matrix s = 0, and x + alpha p
+// solves the system; with a singular one s need not be zero, and the iteration
+// breaks down.  (In every other case a half step that would meet the tolerance
+// ends its iteration with a smaller ||r||, so ||s|| is formed only here.)
+__device__ __forceinline__ void scalars_half_step(KrylovScalars* S, double ss)
 {
-    S->snorm = 0;
-    S->res = 0;
-    S->it += 1;
-    S->status = KS_CONVERGED;
+    S->snorm = sqrt(ss) / S->bnorm;
     S->done = 1;
+    if (S->snorm < S->tol) {
+        S->res = S->snorm;
+        S->it += 1;
+        S->status = KS_CONVERGED;
+    }
+    else {
+        S->res = sqrt(S->rr) / S->bnorm;
+        S->status = KS_BREAKDOWN;
+    }
 }
 
 // WW: compile-time ELL width (0: run-time).  MATS: the CTA's ELL words are
@@ -648,10 +658,13 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
             if (S.done) break;
         }
         if (S.half) {
-            if (!side_x)
-                for (int m = threadIdx.x; m < n; m += T) xp[m] = fma(alpha, sp[m], xp[m]);
-            __syncthreads();
-            if (threadIdx.x == 0) scalars_half_step(&S);
+            R acc[1] = {0};
+            for (int m = threadIdx.x; m < n; m += T) {
+                if (!side_x) xp[m] = fma(alpha, sp[m], xp[m]);
+                acc[0] = fma(ss[m], ss[m], acc[0]);
+            }
+            if (!G.reduce(acc, 2)) return;
+            if (threadIdx.x == 0) scalars_half_step(&S, tot[0]);
             __syncthreads();
             break;
         }

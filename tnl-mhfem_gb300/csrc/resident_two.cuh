@@ -221,9 +221,13 @@ __global__ void __launch_bounds__(kPassThreads, 1) k_bicgstab_two(const Resident
             if (S.done) break;
         }
         if (S.half) {
-            for (int m = threadIdx.x; m < n; m += T) sx[m] = fma(alpha, sp[m], sx[m]);
-            __syncthreads();
-            if (threadIdx.x == 0) scalars_half_step(&S);
+            R acc[1] = {0};
+            for (int m = threadIdx.x; m < n; m += T) {
+                sx[m] = fma(alpha, sp[m], sx[m]);
+                acc[0] = fma(ss[m], ss[m], acc[0]);
+            }
+            if (!G.reduce(acc, 2)) return;
+            if (threadIdx.x == 0) scalars_half_step(&S, tot[0]);
             __syncthreads();
             break;
         }
