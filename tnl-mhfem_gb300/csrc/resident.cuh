@@ -307,26 +307,21 @@ __device__ __forceinline__ void end_of_iteration(KrylovScalars* S, EndLimits* li
         S->rho = rho;
 }
 
-// Whether an iteration of the streamed forms can go without sums over r: from
-// phase B's sums, nothing ends it and it does not restart, by
-// end_of_iteration's conditions with the last known ||r||.  Otherwise it sums,
-// so that every end and restart is decided on the residual itself (r may have
-// vanished, and with it rho').  For a thread beside scalars_omega_beta's: it
-// forms omega and rho' again rather than wait for them.
-__device__ __forceinline__ bool plain_iteration(const KrylovScalars* S, const EndLimits* lim, const double* tot)
+// The end of an iteration of the streamed forms that did not sum over r, with
+// rho' from phase B's sums.  False, and nothing changed, if by end_of_iteration's
+// conditions with the last known ||r|| it may end the solve or restart it: then
+// the sums are formed after all and end_of_iteration decides on the residual
+// itself (r may have vanished, and with it rho').
+__device__ __forceinline__ bool end_unchecked(KrylovScalars* S, const EndLimits* lim, double rho)
 {
-    const double omega = quotient(tot[0], tot[1]), rho = fma(-omega, tot[3], tot[2]);
     const double rho2 = rho * rho, bound2 = lim->restart2 * S->rr;
-    return finite_bits(rho2) && greater_bits(bound2, kTiny) && greater_bits(rho2, bound2) && !zero_bits(omega) &&
-           !zero_bits(S->rho);
-}
-
-// The end of such an iteration.
-__device__ __forceinline__ void end_unchecked(KrylovScalars* S, double rho)
-{
+    if (!finite_bits(rho2) || !greater_bits(bound2, kTiny) || !greater_bits(rho2, bound2) || zero_bits(S->omega) ||
+        zero_bits(S->rho))
+        return false;
     S->it += 1;
     S->restart = 0;
     S->rho = rho;
+    return true;
 }
 
 // What a launch begins with: the scalars of a new solve (or those the last
@@ -431,7 +426,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
     __shared__ KrylovScalars S;
     __shared__ double tot[kSums];
     __shared__ double s_inv_rv, s_rho_next;
-    __shared__ int s_plain;
+    __shared__ int s_sum;
     __shared__ int bad;
     const int T = blockDim.x, rc = g.rc, W = WW > 0 ? WW : g.W;
     const int64_t base = (int64_t)blockIdx.x * rc, rows = g.rows;
@@ -653,7 +648,6 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
             }
             if (!G.reduce(acc, 1)) return;
             if (threadIdx.x == 0 || threadIdx.x == 32) scalars_omega_beta(&S, tot, s_inv_rv, &s_rho_next);
-            else if (!MATS && threadIdx.x == 64) s_plain = plain_iteration(&S, &limits, tot);
             __syncthreads();
             if (S.done) break;
         }
@@ -671,7 +665,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
         // C. r, p (and x, while the sums go round), (r, r), (rh, r) -> convergence, restart
         {
             const R omega = (R)S.omega, beta = (R)S.beta;
-            const bool check = MATS || !s_plain || ((S.it + 1) & g.check_mask) == 0 || k + 1 == g.max_its ||
+            const bool check = MATS || ((S.it + 1) & g.check_mask) == 0 || k + 1 == g.max_its ||
                                S.it + 1 >= S.max_iter;
             R acc[2] = {0, 0};
             R* const rnew = RECOMP ? sr : st;
@@ -695,7 +689,17 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
             }
             else {
                 if (!G.barrier([&](int w) { if (side_x) add_to_x(omega, ss, w, 1); })) return;
-                if (threadIdx.x == 0) end_unchecked(&S, s_rho_next);
+                if (threadIdx.x == 0) s_sum = !end_unchecked(&S, &limits, s_rho_next);
+                __syncthreads();
+                if (s_sum) {
+                    for (int m = threadIdx.x; m < n; m += T) {
+                        const R rv = rnew[m];
+                        acc[0] = fma(rv, rv, acc[0]);
+                        acc[1] = fma(srh[m], rv, acc[1]);
+                    }
+                    if (!G.reduce(acc, 2)) return;
+                    if (threadIdx.x == 0) end_of_iteration(&S, &limits, tot[0], tot[1], k + 1 == g.max_its);
+                }
             }
             if constexpr (!RECOMP) {  // r is where t was; the next s takes its place, the next t that of this s
                 st = ss;
