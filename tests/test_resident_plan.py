@@ -45,6 +45,40 @@ def test_every_launch_is_within_its_kernels_bounds(plan):
             assert (P["ctas"] - 1) * P["rc"] < r, at
 
 
+def _form(P):
+    if not P["ok"]:
+        return "five kernels"
+    if P["two"]:
+        return "cluster" if P["cluster"] else "two"
+    if P["mats"]:
+        return "three, s recomputed" if P["recomp"] else "three"
+    return "streamed" if P["x_in_smem"] else "x in memory"
+
+
+# (rows, width, bytes per value) -> the form that takes the system: the sizes by which the GPU tests
+# reach each form
+FORMS = {
+    (3_960, 4, 8): "cluster", (4_181, 4, 8): "two", (124_033, 4, 8): "two", (126_485, 4, 8): "three, s recomputed",
+    (249_408, 4, 8): "three, s recomputed", (252_880, 4, 8): "three", (357_765, 4, 8): "streamed",
+    (677_825, 4, 8): "x in memory", (812_240, 4, 8): "x in memory", (821_633, 4, 8): "five kernels",
+    (297_714, 6, 8): "streamed", (777_600, 6, 8): "x in memory",
+    (346_560, 9, 8): "streamed", (686_816, 9, 8): "x in memory", (736_400, 9, 8): "five kernels",
+    (382_500, 10, 8): "streamed", (658_800, 10, 8): "five kernels",
+    (196_800, 13, 8): "streamed", (536_256, 13, 8): "five kernels", (312_132, 21, 8): "five kernels",
+    (459_425, 4, 4): "three, s recomputed", (555_560, 4, 4): "streamed", (1_388_560, 4, 4): "x in memory",
+    (1_648_725, 4, 4): "five kernels", (1_626_560, 4, 4): "five kernels",
+    (437_778, 6, 4): "streamed", (1_515_000, 6, 4): "x in memory", (1_703_520, 6, 4): "five kernels",
+    (240_800, 9, 4): "three, s recomputed", (346_560, 9, 4): "streamed", (1_060_080, 9, 4): "five kernels",
+    (227_556, 10, 4): "three, s recomputed", (382_500, 10, 4): "streamed", (957_168, 10, 4): "five kernels",
+    (143_856, 13, 4): "three, s recomputed", (261_360, 13, 4): "streamed", (726_516, 13, 4): "five kernels",
+    (488_136, 21, 4): "five kernels",
+}
+
+
+def test_forms_at_the_sizes_of_the_gpu_tests(plan):
+    assert {k: _form(P) for k, P in zip(FORMS, plan(FORMS))} == FORMS
+
+
 def test_gmres_route_follows_rows_and_width(plan):
     """On the faster side at the sizes where both routes were measured, and resident up to 2^18 rows
     whatever the width."""

@@ -74,6 +74,10 @@ constexpr int64_t kEveryTestRows = (int64_t)1 << 18;
 // takes hundreds of iterations.
 constexpr int kStreamedCheckEvery = 4;
 
+// Shared memory left for the kernels' static variables: the cluster's slots
+// take 2 KB of the two-reduction form's.
+constexpr size_t kStaticTwo = 4096, kStaticThree = 2048;
+
 struct ResidentPlan {
     bool ok = false, cluster = false, mats = false, recomp = false, x_in_smem = false;
     bool two = false;  // resident_two.cuh
@@ -96,7 +100,7 @@ inline ResidentPlan plan_resident(int64_t rows, int width, size_t real, int sms,
                  (P.two    ? (real * (1 + 4 * (size_t)width) + sizeof(int32_t) * width) * P.rc
                   : P.mats ? (real + sizeof(int32_t)) * (size_t)width * P.rc
                            : 0);
-        return P.smem + 4096 <= smem_max;  // 4 KB for the static shared variables
+        return P.smem + (P.two ? kStaticTwo : kStaticThree) <= smem_max;
     };
     const int64_t want = (rows + 127) / 128;
     const int ctas = (int)std::min<int64_t>(want, sms);
