@@ -84,3 +84,24 @@ def test_half_step_that_solves(rows, width):
     st, it, res, x = solve_blocks([[1.0, 0.0], [0.0, 1.0]], [1.0, -1.0], rows, width)
     assert st == L.OK and it == 1 and res == 0
     assert np.array_equal(x, np.tile([1.0, -1.0], (rows // 2, 1)))
+
+
+@pytest.mark.parametrize("rows,width", FORMS)
+def test_breakdown(rows, width):
+    """(rh, A rh) = 0 in the first iteration: no alpha."""
+    st, it, res, x = solve_blocks([[1.0, -3.0], [1.0, 1.0]], [1.0, 1.0], rows, width)
+    assert st == L.ERR_BREAKDOWN and it == 0 and res == 1
+    assert not x.any()
+
+
+# rows of three times a power of two, the forms as above
+@pytest.mark.parametrize("rows,width", [(48, 4), (1536, 6), (12288, 4), (196608, 4), (196608, 6), (196608, 13)])
+def test_restart(rows, width):
+    """The columns of the block sum to 2, so (rh, A s) = 2 (rh, s) = 0 and rho' = 0 after the first
+    iteration (alpha = 1/2, omega = 5, r = (2, -1, -1) / 16): rh = p = r, and the solve goes on.  It
+    could not without the restart: rho = 0 ends it."""
+    block = np.array([[1.0, 0.5, 0.25], [1.0, 1.0, 0.75], [0.0, 0.5, 1.0]])
+    st, it, res, x = solve_blocks(block, [1.0, 1.0, 1.0], rows, width)
+    assert st == L.OK and 2 <= it <= 8 and res < 1e-12
+    # the block's condition number is below 100
+    assert np.abs(x - np.linalg.solve(block, np.ones(3))).max() < 1e-9
