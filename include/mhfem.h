@@ -349,10 +349,10 @@ mhfem_status mhfem_get_stream(mhfem_t h, void** stream);
 mhfem_status mhfem_time_kernel(mhfem_t h, int32_t kernel, int32_t reps, double* ms_per_launch,
                                double* bytes_per_launch, double* flops_per_launch);
 
-/* Check of the bounded grid barrier that the resident solves (BiCGStab and
- * GMRES of systems that fit the SMs) place between their phases.  One cooperative launch of `ctas` CTAs on `device`
- * passes through the barrier once, every wait polling at most `max_polls`
- * times; CTA `skip_cta` (none if negative) never arrives, so the others'
+/* Check of the bounded waits of the resident solves (BiCGStab and GMRES of
+ * systems that fit the SMs).  One cooperative launch of `ctas` CTAs on
+ * `device` goes through one reduction and one barrier of those solves, every
+ * wait polling at most `max_polls` times; CTA `skip_cta` (none if negative) never arrives, so the others'
  * waits run out, set the failure flag and return -- the kernel ends without
  * a fault or a hang and the context stays usable.  Returns the CTAs that
  * passed and that gave up, and the flag (the solve turns it into

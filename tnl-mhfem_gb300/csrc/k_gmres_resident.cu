@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kGmresThreads, 1) k_gmres_resident(const Gmres
                 scol[k * rc + m] = CL ? map_rank(smem_u32(su + c % rc), c / rc) : c;
             }
     }
-    Group<CL> G{col, tot, slots, &bad, g.partials, g.bar, g.bar_err, g.host_wait, g.give_up};
+    Group<CL> G{col, tot, slots, &bad, g.partials, g.bar, g.bar_err, g.host_wait, g.give_up, {}};
     G.begin();
     if constexpr (CL) cluster_barrier();
     else __syncthreads();

@@ -793,22 +793,6 @@ __global__ void __launch_bounds__(KB) k_update_p(int64_t rows, T* p, const T* r,
     }
 }
 
-// ---- check of the bounded grid wait ------------------------------------------------
-
-// Check of the bounded barrier: every CTA but `skip` (none if negative)
-// arrives once and reports 1 (passed) or 0 (gave up); CTA `skip` never
-// arrives and reports -1, so the others' waits run out after max_polls.
-__global__ void __launch_bounds__(KB) k_grid_barrier_check(unsigned int* count, int* err, int skip,
-                                                           unsigned int max_polls, int* result)
-{
-    if ((int)blockIdx.x == skip) {
-        if (threadIdx.x == 0) result[blockIdx.x] = -1;
-        return;
-    }
-    const bool ok = grid_barrier(count, err, gridDim.x, max_polls);
-    if (threadIdx.x == 0) result[blockIdx.x] = ok ? 1 : 0;
-}
-
 // ---- launch shapes ---------------------------------------------------------------
 
 
@@ -1233,43 +1217,6 @@ void krylov_fp64_kernel_once(const EllMatrix& A, KrylovWork& W, int which, cudaS
     };
     if (v2) run(std::integral_constant<int, 2>{});
     else run(std::integral_constant<int, 1>{});
-}
-
-
-// ---- check of the bounded grid wait: host side -----------------------------------
-
-cudaError_t grid_barrier_check(int ctas, int skip, unsigned int max_polls, int* passed, int* gave_up, int* flag)
-{
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    int nb = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_grid_barrier_check, KB, 0);
-    if (e != cudaSuccess) return e;
-    if (ctas < 1 || ctas > nb * sm_count(dev)) return cudaErrorInvalidValue;
-    unsigned int* buf = nullptr;  // [0] arrival count, [1] failure flag, [2 ..] per-CTA results
-    e = cudaMalloc(&buf, sizeof(unsigned int) * (2 + (size_t)ctas));
-    if (e != cudaSuccess) return e;
-    std::vector<int> res((size_t)ctas + 2, 0);
-    e = cudaMemset(buf, 0, sizeof(unsigned int) * (2 + (size_t)ctas));
-    if (e == cudaSuccess) {
-        unsigned int* count = buf;
-        int* err = reinterpret_cast<int*>(buf + 1);
-        int* result = reinterpret_cast<int*>(buf + 2);
-        void* args[] = {(void*)&count, (void*)&err, (void*)&skip, (void*)&max_polls, (void*)&result};
-        e = cudaLaunchCooperativeKernel((const void*)k_grid_barrier_check, dim3(ctas), dim3(KB), args, 0, 0);
-        if (e == cudaSuccess) e = cudaMemcpy(res.data(), buf, sizeof(int) * (2 + (size_t)ctas), cudaMemcpyDeviceToHost);
-    }
-    cudaFree(buf);
-    if (e != cudaSuccess) return e;
-    *passed = 0;
-    *gave_up = 0;
-    for (int b = 0; b < ctas; ++b) {
-        *passed += res[2 + b] == 1;
-        *gave_up += res[2 + b] == 0;
-    }
-    *flag = res[1];
-    return cudaSuccess;
 }
 
 void mixed_apply_correction(double* x, KrylovWork& W, cudaStream_t s)

@@ -371,7 +371,7 @@ __device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int* p)
 // __syncthreads) and its reads after the wait, with no thread fence: 1.5
 // instead of 1.9 us for a barrier over 152 CTAs.
 __device__ __forceinline__ bool arrive_and_wait(unsigned int* count, int* err, unsigned int target,
-                                                unsigned int max_polls = kBarrierPolls)
+                                                unsigned int max_polls)
 {
     asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(count), "r"(1u) : "memory");
     unsigned int polls = 0;
@@ -382,19 +382,6 @@ __device__ __forceinline__ bool arrive_and_wait(unsigned int* count, int* err, u
         }
     }
     return true;
-}
-
-// Arrive at the grid barrier whose cumulative arrival count is `target`
-// (it grows by gridDim.x per barrier) and wait for every CTA.  False (in
-// every thread of the CTA) when the wait gave up.
-__device__ __forceinline__ bool grid_barrier(unsigned int* count, int* err, unsigned int target,
-                                             unsigned int max_polls = kBarrierPolls)
-{
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) ok = arrive_and_wait(count, err, target, max_polls) ? 1 : 0;
-    __syncthreads();
-    return ok != 0;
 }
 
 }  // namespace mhfem

@@ -219,9 +219,9 @@ cudaError_t krylov_resident_fp64(const EllMatrix& A, const double* b, double tol
                                  double* x, KrylovWork& W, KrylovScalars* host, int iters, cudaStream_t s);
 // The same for the mixed form's inner solve, set up by mixed_inner_init.
 cudaError_t krylov_resident_fp32(const EllMatrix& A, KrylovWork& W, KrylovScalars* host, int iters, cudaStream_t s);
-// One cooperative launch of `ctas` CTAs through the persistent solves'
-// bounded grid barrier, CTA `skip` (none if negative) never arriving; counts
-// the CTAs that passed and that gave up, and returns the failure flag.
+// One cooperative launch of `ctas` CTAs through a reduction and a barrier of the
+// resident solves, CTA `skip` (none if negative) never arriving; counts the
+// CTAs that passed and that gave up, and returns the failure flag.
 cudaError_t grid_barrier_check(int ctas, int skip, unsigned int max_polls, int* passed, int* gave_up, int* flag);
 
 // mixed: outer residual r = b - A x (FP64) -> sc; scale into r32; inner FP32 solve; x += scale*e

@@ -123,9 +123,19 @@ __device__ __forceinline__ double lane_sum(const double* col, int lane, int n)
     return (a[0] + a[1]) + (a[2] + a[3]);
 }
 
+// Polls after which a wait gives up: kBarrierPolls in the solves (known when
+// they are compiled), a parameter of the check of the waits.
+struct SolvePolls {
+    __device__ __forceinline__ operator unsigned int() const { return kBarrierPolls; }
+};
+struct CheckPolls {
+    unsigned int polls;
+    __device__ __forceinline__ operator unsigned int() const { return polls; }
+};
+
 // The CTAs of the launch as one group: reductions over all of them and a
 // barrier.  CL: one cluster; else the whole (cooperatively launched) grid.
-template <bool CL>
+template <bool CL, typename Polls = SolvePolls>
 struct Group {
     double* col;     // [kSums][threads]
     double* tot;     // [kSums]
@@ -136,6 +146,7 @@ struct Group {
     int* err;
     int* host_wait;
     int give_up;
+    Polls polls;
     // Arrivals that the counter has seen (in the first warp).  The count runs
     // on from launch to launch: the word behind it holds its value at the last
     // launch's end.
@@ -156,7 +167,7 @@ struct Group {
     // iteration 3 to 4% longer.)
     __device__ __forceinline__ void wait()
     {
-        if (arrive_and_wait(bar, err, target) && (int)blockIdx.x != give_up) return;
+        if (arrive_and_wait(bar, err, target, polls) && (int)blockIdx.x != give_up) return;
         atomicExch(err, 1);
         *bad = 1;
         if (host_wait) *(volatile int*)host_wait = 1;
@@ -463,7 +474,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_bicgstab_resident(const Resi
                 sa[k * rc + m] = __ldg(g.vals + o);
                 scol[k * rc + m] = c;
             }
-    Group<false> G{col, tot, nullptr, &bad, g.partials, g.bar, g.bar_err, g.host_wait, g.give_up};
+    Group<false> G{col, tot, nullptr, &bad, g.partials, g.bar, g.bar_err, g.host_wait, g.give_up, {}};
     G.begin();
     __syncthreads();
 

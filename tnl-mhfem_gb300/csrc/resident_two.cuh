@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(kPassThreads, 1) k_bicgstab_two(const Resident
             ea[k * rc + m] = __ldg(g.vals + o);
             ec[k * rc + m] = CL ? map_rank(smem_u32(sr + c % rc), c / rc) : c;
         }
-    Group<CL> G{col, tot, slots, &bad, g.partials, g.bar, g.bar_err, g.host_wait, g.give_up};
+    Group<CL> G{col, tot, slots, &bad, g.partials, g.bar, g.bar_err, g.host_wait, g.give_up, {}};
     G.begin();
     if constexpr (CL) cluster_barrier();
     else __syncthreads();
