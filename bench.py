@@ -861,7 +861,45 @@ def main():
         "gpu_launches": gpu_launches,
         "clocks": clk,
     }
-    print(json.dumps(line), flush=True)
+    print(json.dumps({"detail": line}), file=sys.stderr, flush=True)
+    print(json.dumps(result_line(line)), flush=True)
+
+
+def rounded(v):
+    """Floats to six digits, through dicts and lists."""
+    if isinstance(v, dict):
+        return {k: rounded(x) for k, x in v.items()}
+    if isinstance(v, (list, tuple)):
+        return [rounded(x) for x in v]
+    return float(f"{v:.6g}") if isinstance(v, float) else v
+
+
+def result_line(line):
+    """The benchmark's line: the contract's keys whole, of every other leg its rate, its iterations,
+    its speedups and its largest error.  A reader may keep only the last few KB of the output, so the
+    per-step and per-kernel lists go to stderr with everything else (one JSON line, key "detail")."""
+    def arm(d):
+        out = {k: d[k] for k in ("value", "iterations_per_step") if k in d}
+        out.update((k, v) for k, v in d.items() if k.startswith("speedup_vs") and isinstance(v, float))
+        err = d.get("rel_err_vs_fp64_1e-13_max")
+        if err:
+            out["max_rel_err"] = err["face_traces"]
+        return out
+
+    out = {k: v for k, v in line.items()
+           if k not in ("iteration_kernels", "kernels", "forms", "other_cells", "other_configs")}
+    out["roofline"] = {k: v for k, v in line["roofline"].items() if k not in ("selection", "other_spmv")}
+    out["kernel_hbm_frac"] = {k: v["hbm_frac"] for k, v in {**line["iteration_kernels"], **line["kernels"]}.items()}
+    forms = dict(line["forms"] or {})
+    protocol = forms.pop("learned_protocol", None)
+    out["forms"] = {k: arm(v) for k, v in forms.items()}
+    if protocol:
+        out["forms"]["learned_protocol"] = {k: v["protocol"]["value"] for k, v in protocol.items()
+                                            if isinstance(v, dict) and "protocol" in v}
+    out["other"] = {k: arm(v) for k, v in (line["other_cells"] or {}).items()}
+    for name, cfg in (line["other_configs"] or {}).items():
+        out["other"][name] = {k: arm(cfg[k]) for k in ("fp64", "mixed") if k in cfg}
+    return rounded(out)
 
 
 def ncu_traffic(kernel_name, grid):
