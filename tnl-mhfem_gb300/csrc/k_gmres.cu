@@ -31,7 +31,8 @@
 //  - every iteration kernel returns at once when the cycle has ended or the
 //    solve is done, so the host replays a CUDA graph of several iterations
 //    between checks;
-//  - systems of at most 3 * 2^18 rows run resident on the SMs instead
+//  - the systems of gmres_resident_fits (up to 3 x 2^18 rows, fewer at larger
+//    widths; resident_plan.h) run resident on the SMs instead
 //    (k_gmres_resident.cu): one launch per chunk of iterations, restarts
 //    included.
 #include <algorithm>

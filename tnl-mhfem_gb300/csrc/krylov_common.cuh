@@ -193,10 +193,10 @@ __device__ __forceinline__ bool ticket_last(uint32_t* counter)
 
 // Deterministic sum of the partials by the last block (fixed order), in out[]
 // of thread 0: every thread issues its (at most four per pass) partial loads
-// together, then warp q adds the threads' sums of value q.  Shuffle trees in
-// every warp and a sum over the warps in every thread, as before, kept the
-// FP64 pipe of the one SM that works here busy for 2,600 cycles per value
-// (1.3 us of every reduction's tail), now 600 and one tree.
+// together, then warp q adds the threads' sums of value q: 600 cycles of the
+// FP64 pipe of the one SM that works here and one shuffle tree (with trees in
+// every warp and a sum over the warps in every thread it was busy for 2,600
+// cycles per value, 1.3 us of every reduction's tail).
 template <int NV>
 __device__ __forceinline__ void final_sums(const double* partials, double (&out)[NV])
 {

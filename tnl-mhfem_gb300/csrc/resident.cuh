@@ -139,7 +139,7 @@ template <bool CL, typename Polls = SolvePolls>
 struct Group {
     double* col;     // [kSums][threads]
     double* tot;     // [kSums]
-    double* slots;   // cluster: [3][kSums][kMaxCluster]
+    double* slots;   // cluster: [kinds of reduction][kSums][kMaxCluster]
     int* bad;        // shared: a wait gave up
     double* partials;
     unsigned int* bar;
