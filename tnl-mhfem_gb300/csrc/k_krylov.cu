@@ -21,7 +21,6 @@
 #include <algorithm>
 #include <initializer_list>
 #include <type_traits>
-#include <vector>
 
 #include "fp_convert.h"
 #include "krylov_common.cuh"
